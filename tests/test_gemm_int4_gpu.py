@@ -135,3 +135,19 @@ def test_bad_arguments_launch_nothing():
     assert b"multiple of 32" in lib.wst_last_error()
     torch.cuda.synchronize()
     assert (host(y) == 7.0).all()
+
+
+@pytest.mark.parametrize("n", [1, 8, 9, 16, 17, 31, 32, 33])
+@pytest.mark.parametrize("in_f,out_f", [(32, 17), (160, 33), (1056, 96), (3584, 2400)])
+def test_few_tokens_at_the_edges_of_the_tiles(in_f, out_f, n):
+    """The kernel for at most 32 tokens: token tiles of 8, 16 and 32 either side of their
+    edges, one group of K, a slab of K that ends inside its four groups, K shorter and
+    longer than the eight warps' slabs, 16- and 32-row tiles cut off at the last row."""
+    qw, si, sb = fast_packed_weights(in_f, out_f, in_f + out_f + n)
+    rng = np.random.default_rng(n + in_f)
+    x = rng.uniform(-1, 1, (n, in_f)).astype(np.float16)
+    b = rng.standard_normal(out_f).astype(np.float16)
+    y0 = rng.standard_normal((n, out_f)).astype(np.float32)
+    got, _ = run(qw, si, sb, x, b, y0, in_f, out_f, True)
+    close(got, orc.gemm_int4_hier(qw, si, sb, x, in_f, out_f, b, y0),
+          3e-3 * max(1.0, (in_f / 896) ** 0.5), f"{in_f} x {out_f} x {n}")

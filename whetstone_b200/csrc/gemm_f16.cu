@@ -30,6 +30,7 @@
 
 #include <initializer_list>
 
+#include "gemm_int4_few.cuh"
 #include "tensor_map.cuh"
 #include "wst_common.cuh"
 #include "wst_ptx.cuh"
@@ -674,6 +675,8 @@ extern "C" wst_status_t wst_gemm_int4_hier(const void *qw, const void *si, const
   if (!device_facts(&facts)) return WST_ERR_CUDA;
   if (facts.cc_major < 10)
     return fail(WST_ERR_UNSUPPORTED_ARCH, "wst_gemm_int4_hier: this library is built for sm_100a only");
+  if (n <= kInt4FewTokens)
+    return launch_gemm_int4_few(qw, si, sb, x, bias, y, in_f, out_f, n, accum, facts.sm_count);
   unsigned int *err_word = device_error_word();
   if (!err_word) return WST_ERR_CUDA;
   GemmArgs a{};
