@@ -480,6 +480,40 @@ def test_paged_verify_ragged_token_counts(verify_kernel_choice):
         assert_close_per_head(got[cu_np[s]:cu_np[s + 1]], want, f"ragged seq {s}")
 
 
+# counts at the edges of a query tile: 18 tokens of 7 heads, 32 tokens of 4 heads
+@pytest.mark.parametrize("shape,lengths,counts", [
+    (workloads.QWEN25_7B, [130, 0, 700, 61], [18, 37, 4, 19]),
+    (workloads.QWEN25_7B, [2500, 1100, 5], [3, 300, 1]),
+    (workloads.QWEN25_7B, [0], [129]),
+    (workloads.QWEN25_05B, [300, 0, 40], [2, 130, 55]),
+    (workloads.QWEN3_8B, [0, 513, 90], [65, 5, 32]),
+])
+def test_paged_prompts_beside_drafts(shape, lengths, counts):
+    """A step in which sequences read more rows than one query tile beside others that verify."""
+    n_q, n_kv, hd, theta = shape.n_q, shape.n_kv, shape.head_dim, 1e6
+    rng = np.random.default_rng(sum(counts))
+    cache, table_np, k_ctx, v_ctx = build_paged_case(rng, shape, lengths, max(counts))
+    n_seq, total = len(counts), sum(counts)
+    cu_np = np.concatenate([[0], np.cumsum(counts)]).astype(np.int32)
+    qkv = workloads.f16_values(rng, (total, shape.qkv_width))
+    qd, pos0, cu = dev(qkv), dev(np.asarray(lengths, np.int32)), dev(cu_np)
+    max_len = max(l + c for l, c in zip(lengths, counts))
+    paged.rope_cache(qd, cache, decode.RopeTable(max_len, hd, theta), n_q, pos0, cu, total)
+    scratch = torch.empty(paged.verify_scratch_floats(n_seq, max(counts), n_q, n_kv, hd, max_len),
+                          dtype=torch.float32, device="cuda")
+    fill_bits(scratch.view(torch.float16), NAN16)
+    out = torch.zeros(total * n_q * hd, dtype=torch.float16, device="cuda")
+    paged.attn_verify(qd, cache, out, scratch, n_q, pos0, cu, total, max(counts), max_len)
+    got = host(out).astype(np.float64).reshape(total, n_q, hd)
+    assert decode.device_error() == 0
+    for s, (L, c) in enumerate(zip(lengths, counts)):
+        qr, kr, vv = orc.rope_append(qkv[cu_np[s]:cu_np[s + 1]], L + np.arange(c), n_q, n_kv, hd, theta)
+        k_all = np.concatenate([k_ctx[s].astype(np.float64).transpose(1, 0, 2), kr])
+        v_all = np.concatenate([v_ctx[s].astype(np.float64).transpose(1, 0, 2), vv])
+        want = orc.attention_blocked(qr, k_all, v_all, L + 1 + np.arange(c))
+        assert_close_per_head(got[cu_np[s]:cu_np[s + 1]], want, f"seq {s} ({L} + {c} rows)")
+
+
 # ------------------------------------------- bounded waits report, never hang
 
 def test_exchange_wait_runs_out_and_reports():

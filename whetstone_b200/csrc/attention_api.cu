@@ -729,9 +729,18 @@ extern "C" wst_status_t wst_attn_verify_paged(const void *qkv, const void *k_poo
     return fail(WST_ERR_SHAPE,
                 "wst_attn_verify_paged: needs head_dim 64 or 128, at most 64 query heads per "
                 "KV head and 16-byte aligned buffers");
-  if (g_kernel_choice.load() != 2 &&
-      prefill_split_supports(n_q, n_kv, head_dim, max_tokens_per_seq)) {
-    /* all query rows of a (sequence, KV head) unit fit one 128-row tcgen05 tile */
+  /* The persistent tcgen05 kernel takes every batch whose items -- (sequence, KV head, tile
+   * of 128 query rows) -- its scratch layout and the merge's grid can hold: beside drafts
+   * that verify, prompts of any number of rows (two of 300 rows beside six of 4 drafts
+   * against 512 to 8192 rows, 28 heads over 4: 91 us per layer with the append, 255 when the
+   * row-block kernel served them). */
+  const int choice = g_kernel_choice.load();
+  const bool one_tile = prefill_split_supports(n_q, n_kv, head_dim, max_tokens_per_seq);
+  const long long verify_floats =
+      wst_attn_verify_scratch_floats(n_seq, max_tokens_per_seq, n_q, n_kv, head_dim, max_len);
+  const bool span = choice != 3 && verify_span_fits(n_seq, max_tokens_per_seq, n_q, n_kv, head_dim,
+                                                    verify_floats);
+  if (choice != 2 && (one_tile || span)) {
     DeviceFacts facts;
     if (!device_facts(&facts)) return WST_ERR_CUDA;
     PrefillLaunch P;
@@ -752,21 +761,15 @@ extern "C" wst_status_t wst_attn_verify_paged(const void *qkv, const void *k_poo
     P.max_seq = max_pages * page_size;
     P.scale = scale;
     P.scratch = static_cast<float *>(scratch);
-    P.scratch_floats =
-        wst_attn_verify_scratch_floats(n_seq, max_tokens_per_seq, n_q, n_kv, head_dim, max_len);
+    P.scratch_floats = verify_floats;
     P.max_len = max_len;
-    /* the span kernel needs room for at least two slices per unit in the scratch
-     * (a tiny batch against a short prefix has less: the sliced schedule takes it) */
-    const long long units = static_cast<long long>(n_seq) * n_kv;
-    const long long slice_floats =
-        units * max_tokens_per_seq * (n_q / n_kv) * (static_cast<long long>(head_dim) + 4);
-    const bool span_fits = (P.scratch_floats - units) / slice_floats >= 2;
-    if (g_kernel_choice.load() != 3 && span_fits) {
-      /* one persistent CTA per SM over equal spans of all units' KV tiles */
+    if (span) {
+      /* one persistent CTA per SM over equal spans of all items' KV tiles */
       P.span_ctas = rows_tuning().verify_ctas;
       return launch_verify_span(P);
     }
-    /* kernel choice 3: one CTA per slice of about 2048 positions (contiguous runs of 16
+    /* kernel choice 3, or a tiny batch against a short prefix whose scratch has no room for
+     * two slices: one CTA per slice of about 2048 positions (contiguous runs of 16
      * tiles), the older schedule: sequences get as many working CTAs as their length
      * asks for; more, shorter slices only when the batch is too small to fill the GPU */
     int splits = facts.sm_count / (n_seq * n_kv);
@@ -798,8 +801,7 @@ extern "C" wst_status_t wst_attn_verify_paged(const void *qkv, const void *k_poo
   L.hd = head_dim;
   L.scale = scale;
   L.scratch = static_cast<float *>(scratch);
-  L.scratch_floats =
-      wst_attn_verify_scratch_floats(n_seq, max_tokens_per_seq, n_q, n_kv, head_dim, max_len);
+  L.scratch_floats = verify_floats;
   L.max_len = max_len;
   L.out = out;
   return launch_rows(L);

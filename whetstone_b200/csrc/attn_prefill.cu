@@ -1011,38 +1011,40 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap kmap,
 }
 
 /* ------------------------------------------------------------------------
- * Ragged paged verify as ONE persistent wave: attn_verify_span_kernel.
+ * Ragged paged batches as ONE persistent wave: attn_verify_span_kernel.
  *
- * The (sequence, KV head) units of a ragged batch differ in length by an order of
- * magnitude, and every unit has a single 128-row query tile (a few draft tokens x the
- * heads of the GQA group).  With one CTA per (unit, slice) each CTA pays a prologue
+ * An item is one tile of up to 128 query rows (tokens x the heads of the GQA group) of a
+ * (sequence, KV head): a handful of draft tokens are one item, a prompt that fills beside
+ * them is many.  Items differ in length by an order of magnitude.  With one CTA per
+ * (item, slice) each CTA pays a prologue
  * (length, page table, first K tile from DRAM, first two score tiles) and an epilogue
  * that nothing else on its SM overlaps, and the last wave is ragged.  Here the KV
- * tiles of ALL units are laid end to end (unit-major) and cut into gridDim.x equal
- * spans; a CTA walks its span, which may cross unit boundaries -- each stretch inside
- * one unit is a "piece" and produces one partial row set (a slice of that unit).  The
+ * tiles of ALL items are laid end to end and cut into gridDim.x equal
+ * spans; a CTA walks its span, which may cross item boundaries -- each stretch inside
+ * one item is a "piece" and produces one partial row set (a slice of that item).  The
  * TMA producer runs ahead across pieces, so the next piece's page ids and first tiles
  * arrive while the current piece is still in its softmax and epilogue; the MMA and
  * softmax warps carry their barrier phases on a tile counter that never restarts.
  * Every CTA streams the same number of tiles (+-1), whatever the lengths are.
  *
  * Same tile pipeline as attn_prefill_kernel (Q and P in tensor memory, two score
- * buffers, two softmax threads per row, lazy rescale); the slices of a unit are
- * merged by attn_merge_kernel, which reads each unit's slice count from the tail of
+ * buffers, two softmax threads per row, lazy rescale); the slices of an item are
+ * merged by attn_merge_rows_kernel, which reads each item's slice count from the tail of
  * the scratch buffer.
  * ---------------------------------------------------------------------- */
 struct SpanArgs {
   const float *q;
   long long q_tok_stride;
-  float *scratch;            /* [unit][max_slices][rows_cap][hd+4], then int32 counts[n_units] */
+  float *scratch;            /* [item][max_slices][rows_cap][hd+4], then int32 counts[n_items] */
   int *slice_counts;
   const int32_t *pos0_dev;   /* [n_seq] */
   const int32_t *cu_tokens;  /* [n_seq + 1] */
   const int32_t *page_table; /* [n_seq][max_pages] */
   int max_pages, n_pool_pages;
   int n_seq, n_q, n_kv, gqa, max_seq;
+  int n_tok, tpt, n_qtiles; /* tokens of a sequence at most, tokens of a query tile, tiles of n_tok */
   int max_slices, rows_cap;
-  int min_span; /* tiles: no unit may be cut into more than max_slices pieces */
+  int min_span; /* tiles: no item may be cut into more than max_slices pieces */
   int early;    /* the batch description and the cache rows below every sequence's new
                  * tokens are not written by the launch ahead: read them before the grid
                  * dependency resolves */
@@ -1050,64 +1052,73 @@ struct SpanArgs {
   unsigned int *err_word;
 };
 
-/* One stretch of a CTA's span inside one unit. */
+/* One stretch of a CTA's span inside one item. */
 struct SpanPiece {
-  int seq, kvh, first, n, slice, count; /* count > 0 only on the unit's first piece */
-  int pos0, tok_begin, ntok, kv_end;
+  int seq, kvh, qt, first, n, slice, count; /* count > 0 only on the item's first piece */
+  int pos0;                                 /* cache rows the sequence had before this step */
+  int q_pos0, tok_begin, ntok, kv_end;      /* of the item's query tile */
 };
 
-/* What starting a piece costs a CTA, in tiles: the next unit's q has to be fetched and
+/* What starting a piece costs a CTA, in tiles: the next item's q has to be fetched and
  * staged and the pipeline refilled while the finished piece's rows are stored (measured:
- * 4 to 5 us per unit boundary against 1.8 us per tile).  The span arithmetic counts every
- * unit as kUnitPad + tiles "slots", so a span with many short units gets fewer real
- * tiles than one inside a long unit, and all CTAs finish together. */
+ * 4 to 5 us per item boundary against 1.8 us per tile).  The span arithmetic counts every
+ * item as kUnitPad + tiles "slots", so a span with many short items gets fewer real
+ * tiles than one inside a long item, and all CTAs finish together. */
 constexpr int kUnitPad = 3;
 
 /* Walks the pieces of a span; every role of the CTA runs its own copy.  Positions are
- * slots: unit u owns slots [start_u, start_u + kUnitPad + tiles_u); the first kUnitPad
- * of them are padding, slot kUnitPad + i is KV tile i. */
+ * slots: an item of t tiles owns slots [start, start + kUnitPad + t); the first kUnitPad
+ * of them are padding, slot kUnitPad + i is KV tile i.  Items lie sequence by sequence,
+ * in a sequence KV head by KV head, the query tiles of a head one after the other: the
+ * CTAs that share a head's K and V in L2 run at the same time. */
 struct SpanWalk {
-  int seq, kvh, slot; /* where the next piece starts: slot index inside the unit */
-  long long g, hi;    /* global slot index of that point, end of the span */
-  long long before;   /* slots of all units of earlier sequences */
+  int seq, kvh, qt, slot; /* where the next piece starts: slot index inside the item */
+  long long g, hi;        /* global slot index of that point, end of the span */
+  long long start;        /* global slot index of the item's first slot */
   int span, cta;
   const SpanArgs *a;
 
-  __device__ __forceinline__ static int seq_tiles(const SpanArgs &a, int s, int *pos0, int *tok_begin,
-                                                  int *ntok, int *kv_end) {
-    const int b = a.cu_tokens[s];
-    const int n = a.cu_tokens[s + 1] - b;
-    const int p0 = max(a.pos0_dev[s], 0);
-    const int end = n > 0 ? min(p0 + n, a.max_seq) : 0;
-    *pos0 = p0;
-    *tok_begin = b;
-    *ntok = n;
-    *kv_end = end;
-    return (end + 127) / 128;
+  __device__ __forceinline__ static int seq_tokens(const SpanArgs &a, int s) {
+    return min(a.cu_tokens[s + 1] - a.cu_tokens[s], a.n_tok);
   }
-  /* slots of one unit of a sequence with t tiles (0 for a sequence without tokens) */
-  __device__ __forceinline__ static int unit_slots(int t) { return t > 0 ? t + kUnitPad : 0; }
+  /* KV tiles that a sequence's query tile sees: all up to its own last token */
+  __device__ __forceinline__ static int item_end(const SpanArgs &a, int pos0, int n, int qt) {
+    return min(pos0 + min((qt + 1) * a.tpt, n), a.max_seq);
+  }
+  /* slots of one KV head of a sequence (0 for a sequence without tokens) */
+  __device__ __forceinline__ static long long head_slots(const SpanArgs &a, int s) {
+    const int n = seq_tokens(a, s), pos0 = max(a.pos0_dev[s], 0);
+    long long sum = 0;
+    for (int qt = 0; qt * a.tpt < n; ++qt) sum += (item_end(a, pos0, n, qt) + 127) / 128 + kUnitPad;
+    return sum;
+  }
 
   __device__ __forceinline__ bool next(SpanPiece *p) {
     while (g < hi && seq < a->n_seq) {
-      const int t = seq_tiles(*a, seq, &p->pos0, &p->tok_begin, &p->ntok, &p->kv_end);
-      if (t == 0) { /* a sequence without tokens in this step */
+      const int n_seq_tok = seq_tokens(*a, seq);
+      if (n_seq_tok <= 0) { /* a sequence without tokens in this step */
         ++seq;
         continue;
       }
-      const int us = unit_slots(t);
-      const long long left = hi - g;
-      const int n_slots = static_cast<int>(min(static_cast<long long>(us - slot), left));
-      const long long unit_start = before + static_cast<long long>(kvh) * us;
+      const int tok0 = qt * a->tpt;
+      p->pos0 = max(a->pos0_dev[seq], 0);
+      p->q_pos0 = p->pos0 + tok0;
+      p->tok_begin = a->cu_tokens[seq] + tok0;
+      p->ntok = min(a->tpt, n_seq_tok - tok0);
+      p->kv_end = item_end(*a, p->pos0, n_seq_tok, qt);
+      const int t = (p->kv_end + 127) / 128;
+      const int us = t + kUnitPad;
+      const int n_slots = static_cast<int>(min(static_cast<long long>(us - slot), hi - g));
       /* the real tiles among slots [slot, slot + n_slots) */
       const int first = max(slot - kUnitPad, 0);
       const int last = slot + n_slots - kUnitPad; /* one past */
       const int n = max(last - first, 0);
-      /* slices are numbered by the CTAs that hold real tiles of the unit: the first real
-       * tile sits at unit_start + kUnitPad */
-      const long long first_real = unit_start + kUnitPad;
+      /* slices are numbered by the CTAs that hold real tiles of the item: the first real
+       * tile sits at start + kUnitPad */
+      const long long first_real = start + kUnitPad;
       p->seq = seq;
       p->kvh = kvh;
+      p->qt = qt;
       p->first = first;
       p->n = n;
       p->slice = cta - static_cast<int>(first_real / span);
@@ -1118,10 +1129,13 @@ struct SpanWalk {
       slot += n_slots;
       if (slot == us) {
         slot = 0;
-        if (++kvh == a->n_kv) {
-          kvh = 0;
-          before += static_cast<long long>(a->n_kv) * us;
-          ++seq;
+        start += us;
+        if ((++qt) * a->tpt >= n_seq_tok) {
+          qt = 0;
+          if (++kvh == a->n_kv) {
+            kvh = 0;
+            ++seq;
+          }
         }
       }
       if (n > 0) return true; /* a stretch of padding only is no piece */
@@ -1203,14 +1217,13 @@ attn_verify_span_kernel(const __grid_constant__ CUtensorMap kmap,
    * waits for the dependency right before it first touches what the append writes. */
   if (!a.early) grid_dependency_wait();
 
-  /* ---- where does this CTA's span start?  warp 0: total tiles, span length, and the
-   * (sequence, KV head, tile) at global tile index cta * span */
+  /* ---- where does this CTA's span start?  warp 0: total slots, span length, and the
+   * (sequence, KV head, query tile, slot) at global slot index cta * span */
   if (warp == 0) {
-    int pos0, tb, nt, ke;
     long long total = 0;
     for (int s0 = 0; s0 < a.n_seq; s0 += 32) {
       const int s = s0 + lane;
-      long long t = s < a.n_seq ? SpanWalk::unit_slots(SpanWalk::seq_tiles(a, s, &pos0, &tb, &nt, &ke)) : 0;
+      long long t = s < a.n_seq ? SpanWalk::head_slots(a, s) : 0;
 #pragma unroll
       for (int off = 16; off > 0; off >>= 1) t += __shfl_xor_sync(0xffffffffu, t, off);
       total += t;
@@ -1220,45 +1233,50 @@ attn_verify_span_kernel(const __grid_constant__ CUtensorMap kmap,
     if (span < a.min_span) span = a.min_span;
     const long long lo = static_cast<long long>(blockIdx.x) * span;
     const long long hi = min(lo + span, total);
-    /* the sequence that holds global tile `lo` */
-    long long before = 0;
-    int seq = a.n_seq, kvh = 0, tile = 0;
+    /* the sequence that holds global slot `lo` */
+    long long start = 0;
+    int seq = a.n_seq, kvh = 0, qt = 0, slot = 0;
     if (lo < total) {
       for (int s0 = 0; s0 < a.n_seq && seq == a.n_seq; s0 += 32) {
         const int s = s0 + lane;
-        const long long mine =
-            s < a.n_seq ? static_cast<long long>(a.n_kv) *
-                              SpanWalk::unit_slots(SpanWalk::seq_tiles(a, s, &pos0, &tb, &nt, &ke))
-                        : 0;
+        const long long head = s < a.n_seq ? SpanWalk::head_slots(a, s) : 0;
+        const long long mine = a.n_kv * head;
         long long incl = mine;
 #pragma unroll
         for (int off = 1; off < 32; off <<= 1) {
           const long long up = __shfl_up_sync(0xffffffffu, incl, off);
           if (lane >= off) incl += up;
         }
-        const bool here = mine > 0 && before + incl - mine <= lo && lo < before + incl;
+        const bool here = mine > 0 && start + incl - mine <= lo && lo < start + incl;
         const unsigned vote = __ballot_sync(0xffffffffu, here);
         if (vote) {
           const int src = __ffs(vote) - 1;
-          const long long start = __shfl_sync(0xffffffffu, before + incl - mine, src);
-          const long long t = __shfl_sync(0xffffffffu, mine, src) / a.n_kv;
+          start = __shfl_sync(0xffffffffu, start + incl - mine, src);
+          const long long per_head = __shfl_sync(0xffffffffu, head, src);
           seq = s0 + src;
-          kvh = static_cast<int>((lo - start) / t);
-          tile = static_cast<int>((lo - start) % t);
-          before = start;
+          kvh = static_cast<int>((lo - start) / per_head);
+          start += kvh * per_head;
+          const int n = SpanWalk::seq_tokens(a, seq), pos0 = max(a.pos0_dev[seq], 0);
+          for (;; ++qt) { /* ends: lo lies below the head's last slot */
+            const int us = (SpanWalk::item_end(a, pos0, n, qt) + 127) / 128 + kUnitPad;
+            if (lo < start + us || (qt + 1) * a.tpt >= n) break;
+            start += us;
+          }
+          slot = static_cast<int>(lo - start);
         } else {
-          before += __shfl_sync(0xffffffffu, incl, 31);
+          start += __shfl_sync(0xffffffffu, incl, 31);
         }
       }
     }
     if (lane == 0) {
       walk0[0] = seq;
       walk0[1] = kvh;
-      walk0[2] = tile;
+      walk0[2] = slot;
       walk0[3] = span;
       walk0[4] = lo;
       walk0[5] = hi;
-      walk0[6] = before;
+      walk0[6] = start;
+      walk0[7] = qt;
     }
   }
   tc_fence_before_sync();
@@ -1269,11 +1287,12 @@ attn_verify_span_kernel(const __grid_constant__ CUtensorMap kmap,
   SpanWalk walk;
   walk.seq = static_cast<int>(walk0[0]);
   walk.kvh = static_cast<int>(walk0[1]);
+  walk.qt = static_cast<int>(walk0[7]);
   walk.slot = static_cast<int>(walk0[2]);
   walk.span = static_cast<int>(walk0[3]);
   walk.g = walk0[4];
   walk.hi = walk0[5];
-  walk.before = walk0[6];
+  walk.start = walk0[6];
   walk.cta = static_cast<int>(blockIdx.x);
   walk.a = &a;
   int n_total = 0; /* KV tiles of this CTA (its span minus the padding slots) */
@@ -1519,8 +1538,8 @@ attn_verify_span_kernel(const __grid_constant__ CUtensorMap kmap,
         for (int b = 0; b < OC * 4; b += 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(qn + b));
       }
       const int rows_valid = pc.ntok * a.gqa;
-      const int lim = r < rows_valid ? min(pc.pos0 + r / a.gqa + 1, a.max_seq) : pc.kv_end;
-      const int lim_min = min(pc.pos0 + 1, a.max_seq);
+      const int lim = r < rows_valid ? min(pc.q_pos0 + r / a.gqa + 1, a.max_seq) : pc.kv_end;
+      const int lim_min = min(pc.q_pos0 + 1, a.max_seq);
       const bool live = wq * 32 < rows_valid;
       float m_ref = -INFINITY, l_run = 0.f;
 
@@ -1633,10 +1652,10 @@ attn_verify_span_kernel(const __grid_constant__ CUtensorMap kmap,
         l_run += slot[(half ^ 1) * 128 + r];
         pair_sync(); /* both halves have read before the next piece writes the slot */
       }
-      const long long unit = static_cast<long long>(pc.seq) * a.n_kv + pc.kvh;
+      const long long item = (static_cast<long long>(pc.seq) * a.n_kv + pc.kvh) * a.n_qtiles + pc.qt;
       if (ok && live) {
         tc_fence_after_sync();
-        float *dst = a.scratch + ((unit * a.max_slices + pc.slice) * a.rows_cap + r) * (HD + 4) + half * OC;
+        float *dst = a.scratch + ((item * a.max_slices + pc.slice) * a.rows_cap + r) * (HD + 4) + half * OC;
 #pragma unroll
         for (int c0 = 0; c0 < OC; c0 += 32) {
           uint32_t v[32];
@@ -1651,7 +1670,7 @@ attn_verify_span_kernel(const __grid_constant__ CUtensorMap kmap,
         if (half == 0 && r < rows_valid)
           *reinterpret_cast<float2 *>(dst + HD) = make_float2(m_ref, l_run);
       }
-      if (pc.count > 0 && threadIdx.x == 0) a.slice_counts[unit] = pc.count;
+      if (pc.count > 0 && threadIdx.x == 0) a.slice_counts[item] = pc.count;
       tc_fence_before_sync();
       mbar_arrive(bar(EPI_DONE)); /* O may be overwritten */
       pc = nxt;
@@ -1723,6 +1742,28 @@ bool prefill_kernel_supports(int n_q, int n_kv, int hd, int n) {
   return static_cast<long long>(n) * gqa >= 64;
 }
 
+namespace {
+/* The items of a ragged batch as the span kernel and its merge number them. */
+struct SpanItems {
+  int tpt, n_qtiles; /* tokens per query tile, tiles of the longest sequence */
+  long long count;
+};
+SpanItems span_items(int n_seq, int n_tok_max, int n_q, int n_kv) {
+  SpanItems it;
+  const int fit = 128 / (n_q / n_kv);
+  it.tpt = n_tok_max < fit ? n_tok_max : fit;
+  it.n_qtiles = (n_tok_max + it.tpt - 1) / it.tpt;
+  it.count = static_cast<long long>(n_seq) * n_kv * it.n_qtiles;
+  return it;
+}
+}  // namespace
+
+bool verify_span_fits(int n_seq, int n_tok_max, int n_q, int n_kv, int hd, long long scratch_floats) {
+  if ((hd != 64 && hd != 128) || n_q / n_kv > 128) return false;
+  const SpanItems it = span_items(n_seq, n_tok_max, n_q, n_kv);
+  const long long slice_floats = it.count * it.tpt * (n_q / n_kv) * (static_cast<long long>(hd) + 4);
+  return it.count <= 65535 && (scratch_floats - it.count) / slice_floats >= 2;
+}
 
 wst_status_t launch_verify_span(const PrefillLaunch &P) {
   DeviceFacts facts;
@@ -1733,10 +1774,11 @@ wst_status_t launch_verify_span(const PrefillLaunch &P) {
       !aligned16(P.scratch))
     return fail(WST_ERR_INVALID_ARG, "%s: buffers must be 16-byte aligned", P.name);
   const int gqa = P.n_q / P.n_kv;
-  const int rows_cap = P.n * gqa;
-  const long long units = static_cast<long long>(P.n_seq) * P.n_kv;
+  const SpanItems it = span_items(P.n_seq, P.n, P.n_q, P.n_kv);
+  const int n_qtiles = it.n_qtiles, rows_cap = it.tpt * gqa;
+  const long long units = it.count;
   const long long row_floats = static_cast<long long>(rows_cap) * (P.hd + 4);
-  /* slices a unit may be cut into: what the scratch holds (after it, one count per unit) */
+  /* slices an item may be cut into: what the scratch holds (after it, one count per item) */
   long long cap = (P.scratch_floats - units) / (units * row_floats);
   if (cap > kRowsMaxSplits) cap = kRowsMaxSplits;
   if (cap < 2) return fail(WST_ERR_INVALID_ARG, "%s: scratch too small", P.name);
@@ -1758,12 +1800,17 @@ wst_status_t launch_verify_span(const PrefillLaunch &P) {
   a.n_kv = P.n_kv;
   a.gqa = gqa;
   a.max_seq = P.max_seq;
+  a.n_tok = P.n;
+  a.tpt = it.tpt;
+  a.n_qtiles = n_qtiles;
   a.max_slices = static_cast<int>(cap);
   a.rows_cap = rows_cap;
   a.min_span = (max_tiles + static_cast<int>(cap) - 2) / (static_cast<int>(cap) - 1);
   if (a.min_span < 1) a.min_span = 1;
   a.qscale = P.scale * kLog2e;
-  a.early = decode_overlap_allowed() ? 1 : 0;
+  /* (the early requests are worth two microseconds of a verify step and nothing beside a
+   * prompt's: those batches wait) */
+  a.early = decode_overlap_allowed() && n_qtiles == 1 ? 1 : 0;
   a.err_word = device_error_word();
   if (!a.err_word) return WST_ERR_CUDA;
 
@@ -1804,8 +1851,8 @@ wst_status_t launch_verify_span(const PrefillLaunch &P) {
   m.hd = P.hd;
   m.n_splits = static_cast<int>(cap);
   m.slice_counts = a.slice_counts;
-  m.n_rowblk = 1;
-  m.tpb = P.n;
+  m.n_rowblk = n_qtiles;
+  m.tpb = it.tpt;
   m.rows_cap = rows_cap;
   m.n_units = static_cast<int>(units);
   m.name = P.name;

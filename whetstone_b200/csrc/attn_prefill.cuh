@@ -52,9 +52,13 @@ bool prefill_split_supports(int n_q, int n_kv, int hd, int n_tok_max);
 
 wst_status_t launch_prefill(const PrefillLaunch &P);
 
-/* Ragged paged verify (every unit's query rows in one 128-row tile, prefill_split_supports):
- * the KV tiles of all (sequence, KV head) units end to end, cut into one equal span per
- * persistent CTA, + the slice-merge kernel.  Needs P.page_table, P.cu_tokens, P.pos0_dev,
+/* True if launch_verify_span takes the batch: room for at least two slices of every item
+ * (sequence, KV head, tile of 128 query rows) in `scratch_floats`, and no more items than
+ * the merge kernel's grid has rows. */
+bool verify_span_fits(int n_seq, int n_tok_max, int n_q, int n_kv, int hd, long long scratch_floats);
+
+/* Ragged paged batch, a few drafts or whole prompts per sequence: the KV tiles of all
+ * items end to end, cut into one equal span per persistent CTA, + the slice-merge kernel.  Needs P.page_table, P.cu_tokens, P.pos0_dev,
  * P.scratch and P.max_len. */
 wst_status_t launch_verify_span(const PrefillLaunch &P);
 
