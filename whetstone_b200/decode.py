@@ -21,13 +21,15 @@ _CUDA_STREAM_LEGACY = 0x1  # cudaStreamLegacy: torch's default stream reports ha
 
 def use_torch_stream() -> None:
     """Enqueue this thread's wst_* calls on torch's current CUDA stream, so that
-    torch ops and the kernels are ordered without extra synchronisation."""
-    handle = torch.cuda.current_stream().cuda_stream
-    check(lib.wst_b200_set_stream(ctypes.c_void_p(handle if handle else _CUDA_STREAM_LEGACY)))
+    torch ops and the kernels are ordered without extra synchronisation.  Every wrapper
+    calls this, so it asks torch for the raw handle of the current device's stream: building
+    a torch.cuda.Stream object around it cost 3.2 of a small call's 10.4 us on the host."""
+    handle = torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+    check(lib.wst_b200_set_stream(handle or _CUDA_STREAM_LEGACY))
 
 
-def _ptr(t: torch.Tensor | None) -> ctypes.c_void_p:
-    return ctypes.c_void_p(0 if t is None else t.data_ptr())
+def _ptr(t: torch.Tensor | None) -> int:
+    return 0 if t is None else t.data_ptr()
 
 
 def _require_cuda(t: torch.Tensor, what: str, dtype: torch.dtype) -> None:
@@ -134,7 +136,7 @@ class QkNorm:
 
 def norm_ptrs(qk: QkNorm | None):
     if qk is None:
-        return ctypes.c_void_p(0), ctypes.c_void_p(0), 0.0
+        return None, None, 0.0
     return _ptr(qk.q), _ptr(qk.k), float(qk.eps)
 
 
