@@ -190,3 +190,18 @@ def test_projection_replays_in_a_graph():
     torch.cuda.synchronize()
     close(host(y), orc.gemm_fp16(host(w), x2), 2e-4, "graph replay")
     assert decode.device_error() == 0
+
+
+# (feature tile the dispatch takes: 64, 128, 256, 256 with several tiles per cluster)
+@pytest.mark.parametrize("in_f,out_f,n", [(136, 1001, 129), (72, 64, 256), (200, 4600, 400), (264, 6100, 600),
+                                          (128, 6144, 2048), (40, 9000, 1025)])
+def test_more_than_128_tokens_at_the_edges_of_the_tiles(in_f, out_f, n):
+    """The two-SM tiles: a token or feature tile cut off, K shorter than a stage or ending
+    inside one, columns that vector stores cannot take, both output forms."""
+    rng = np.random.default_rng(in_f + out_f + n)
+    w = (rng.standard_normal((out_f, in_f)) / np.sqrt(in_f)).astype(np.float16)
+    x = rng.standard_normal((n, in_f)).astype(np.float16)
+    b = rng.standard_normal(out_f).astype(np.float16)
+    y0 = rng.standard_normal((n, out_f)).astype(np.float32)
+    close(run(w, x, b, y0, True), orc.gemm_fp16(w, x, b, y0), 2e-4, f"{in_f} x {out_f} x {n}, accumulating")
+    close(run(w, x, None, None, False), orc.gemm_fp16(w, x), 2e-4, f"{in_f} x {out_f} x {n}")

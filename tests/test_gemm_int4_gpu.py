@@ -151,3 +151,19 @@ def test_few_tokens_at_the_edges_of_the_tiles(in_f, out_f, n):
     got, _ = run(qw, si, sb, x, b, y0, in_f, out_f, True)
     close(got, orc.gemm_int4_hier(qw, si, sb, x, in_f, out_f, b, y0),
           3e-3 * max(1.0, (in_f / 896) ** 0.5), f"{in_f} x {out_f} x {n}")
+
+
+# scale bytes that four-byte copies cannot take (3, 5 and 9 groups a row), and those they can
+@pytest.mark.parametrize("in_f,out_f,n", [(96, 1001, 129), (32, 64, 256), (160, 4600, 400), (288, 6100, 600),
+                                          (128, 6144, 2048), (1152, 300, 257)])
+def test_more_than_128_tokens_at_the_edges_of_the_tiles(in_f, out_f, n):
+    """The two-SM tiles with each feature tile (64, 128, 256), K shorter than a stage or ending
+    inside one, one and several tiles per cluster."""
+    qw, si, sb = fast_packed_weights(in_f, out_f, in_f + out_f + n)
+    rng = np.random.default_rng(n + in_f)
+    x = rng.uniform(-1, 1, (n, in_f)).astype(np.float16)
+    b = rng.standard_normal(out_f).astype(np.float16)
+    y0 = rng.standard_normal((n, out_f)).astype(np.float32)
+    got, _ = run(qw, si, sb, x, b, y0, in_f, out_f, True)
+    close(got, orc.gemm_int4_hier(qw, si, sb, x, in_f, out_f, b, y0),
+          3e-3 * max(1.0, (in_f / 896) ** 0.5), f"{in_f} x {out_f} x {n}")

@@ -15,9 +15,8 @@
  *   of the next; persistent CTAs, one per SM, walk the tiles token-tile fastest so
  *   that the CTAs running at the same time share a weight tile in L2.
  *
- *   BN = 256 for real chunks (A 4 KB + B 8 KB of shared memory per 128-clock MMA,
- *   96 bytes per clock); BN = 32, 48 or 64 when the token count is small and the
- *   launch is a stream of the weights: as many CTAs as there are SMs pull on HBM.
+ *   BN = 32, 48 or 64: up to 128 tokens the launch is a stream of the weights, and as
+ *   many CTAs as there are SMs pull on HBM.  More tokens go to gemm_pair.cu.
  *
  * Products are exact in fp32 and accumulated in fp32 (the engine's kernel rounds
  * every group of four products to fp16 first): results differ from the engine's by
@@ -31,6 +30,7 @@
 #include <initializer_list>
 
 #include "gemm_int4_few.cuh"
+#include "gemm_pair.cuh"
 #include "tensor_map.cuh"
 #include "wst_common.cuh"
 #include "wst_ptx.cuh"
@@ -55,7 +55,7 @@ struct GCfg {
   static constexpr int OFF_BAR = NSTAGE * STAGE_BYTES;
   static constexpr int NBAR = 2 * NSTAGE + 4;
   static constexpr int SMEM_BYTES = OFF_BAR + NBAR * 8 + 16 + 1024;
-  static constexpr int ACC_STRIDE = BN <= 32 ? 32 : BN <= 64 ? 64 : 256; /* columns per accumulator */
+  static constexpr int ACC_STRIDE = BN <= 32 ? 32 : 64; /* columns per accumulator */
   static constexpr int TMEM_COLS = 2 * ACC_STRIDE;
   static_assert(RB % 8 == 0 && NSTAGE >= 2, "stage geometry");
   /* the M = 128 read of the last slab of the last stage stays inside the ring */
@@ -68,106 +68,19 @@ struct GemmArgs {
   int in_f, out_f, n, accum;
   int m_tiles, n_tiles;
   unsigned int *err_word;
-  /* the fused form (ROPE): the tile's columns are whole heads of the qkv row; they are
-   * normed, rotated and stored where the attention reads them instead of going to y */
   /* the int4 form (INT4): the weights come packed, one 16-byte word of 32 nibbles and one
    * byte of two 4-bit scale indices per group of 32 along K, one (d, dmin) pair per row */
   const uint4 *qw;       /* [out_f][in_f / 32] */
   const uint8_t *si;     /* [out_f][in_f / 32]: ls | lm << 4 */
   const __half2 *sb;     /* [out_f]: (d, dmin) */
-  __half *q_out;         /* [n][n_q * hd] */
-  __half *k_cache;       /* [n_seq][n_kv][max_seq][hd] */
-  __half *v_cache;
-  const float *cos_tab;  /* [table_len][hd / 2] */
-  const float *sin_tab;
-  const __half *q_gain;  /* [hd] or null */
-  const __half *k_gain;
-  const int32_t *seq_pos0; /* [n_seq] */
-  int n_q, n_kv, hd, n_per_seq, max_seq, table_len;
-  float eps;
 };
-
-/* Epilogue of the fused form for one head of one token: HD accumulator columns from
- * tensor memory (+ bias) -> per-head RMS norm with fp16 gains (q and k heads, if gains
- * are given) -> half-rotation RoPE at the token's position -> fp16, to the q buffer or
- * to the token's cache row; v heads are narrowed and stored as they are.  The
- * arithmetic is that of rope_append_kernel (norm before rotation, x * inv * gain,
- * cuda/decode.cu:112-178 and cuda/chunk_ops.cu:101-150 of the engine). */
-template <int HD>
-__device__ __forceinline__ void rope_head_epilogue(const GemmArgs &a, uint32_t tmem_head, int head,
-                                                   int tpos, long long kv_row, int tok, bool valid) {
-  float x[HD];
-#pragma unroll
-  for (int c0 = 0; c0 < HD; c0 += 32) {
-    uint32_t v[32];
-    tmem_ld_32x32(tmem_head + c0, v);
-    tmem_ld_wait();
-#pragma unroll
-    for (int e = 0; e < 32; ++e) x[c0 + e] = __uint_as_float(v[e]);
-  }
-  if (!valid) return;
-  if (a.bias) {
-#pragma unroll
-    for (int e = 0; e < HD; e += 2) {
-      const float2 b = __half22float2(*reinterpret_cast<const __half2 *>(a.bias + head * HD + e));
-      x[e] += b.x;
-      x[e + 1] += b.y;
-    }
-  }
-  constexpr int HALF = HD / 2;
-  const bool is_q = head < a.n_q, is_k = !is_q && head < a.n_q + a.n_kv;
-  __half *dst;
-  if (is_q) {
-    dst = a.q_out + (static_cast<long long>(tok) * a.n_q + head) * HD;
-  } else {
-    const int kvh = is_k ? head - a.n_q : head - a.n_q - a.n_kv;
-    dst = (is_k ? a.k_cache : a.v_cache) + kv_row + static_cast<long long>(kvh) * a.max_seq * HD;
-  }
-  if (is_q || is_k) {
-    const __half *gain = is_q ? a.q_gain : a.k_gain;
-    if (gain) {
-      float ss = 0.f;
-#pragma unroll
-      for (int e = 0; e < HALF; ++e) ss = fmaf(x[e], x[e], fmaf(x[e + HALF], x[e + HALF], ss));
-      const float inv = rsqrtf(ss / static_cast<float>(HD) + a.eps);
-#pragma unroll
-      for (int e = 0; e < HD; e += 2) {
-        const float2 g = __half22float2(*reinterpret_cast<const __half2 *>(gain + e));
-        x[e] = x[e] * inv * g.x;
-        x[e + 1] = x[e + 1] * inv * g.y;
-      }
-    }
-    const float4 *ct = reinterpret_cast<const float4 *>(a.cos_tab + static_cast<long long>(tpos) * HALF);
-    const float4 *st = reinterpret_cast<const float4 *>(a.sin_tab + static_cast<long long>(tpos) * HALF);
-#pragma unroll
-    for (int e = 0; e < HALF; e += 4) {
-      const float4 c = __ldg(ct + e / 4), sn = __ldg(st + e / 4);
-      const float cc[4] = {c.x, c.y, c.z, c.w}, ss4[4] = {sn.x, sn.y, sn.z, sn.w};
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const float x1 = x[e + k], x2 = x[e + k + HALF];
-        x[e + k] = x1 * cc[k] - x2 * ss4[k];
-        x[e + k + HALF] = x2 * cc[k] + x1 * ss4[k];
-      }
-    }
-  }
-#pragma unroll
-  for (int e = 0; e < HD; e += 8) {
-    uint4 o;
-    o.x = pack_half2(x[e], x[e + 1]);
-    o.y = pack_half2(x[e + 2], x[e + 3]);
-    o.z = pack_half2(x[e + 4], x[e + 5]);
-    o.w = pack_half2(x[e + 6], x[e + 7]);
-    *reinterpret_cast<uint4 *>(dst + e) = o;
-  }
-}
 
 /* Threads of a CTA: 4 epilogue warps, the MMA warp, the TMA warp, and for the int4 form
  * sixteen warps that unpack the weight tile into shared memory. */
 constexpr int kUnpackThreads = 512;
 constexpr int gemm_threads(bool int4) { return int4 ? 192 + kUnpackThreads : 192; }
 
-template <int BN, int KS, int RB, bool ROPE, bool INT4>
+template <int BN, int KS, int RB, bool INT4>
 __global__ void __launch_bounds__(gemm_threads(INT4), 1)
 gemm_f16_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap,
                 const GemmArgs a) {
@@ -408,36 +321,6 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant_
       if (!mbar_wait_idle(bar(ACC_FULL + buf), (local >> 1) & 1, a.err_word, 0x604u)) break;
       tc_fence_after_sync();
       const int row = m0 + r;
-      if constexpr (ROPE) {
-        /* the token's sequence, cache position (clamped, never trusted) and cache row */
-        const bool valid = row < a.n;
-        const int sq = valid ? row / a.n_per_seq : 0;
-        int pos = valid ? a.seq_pos0[sq] + (row - sq * a.n_per_seq) : 0;
-        pos = pos < 0 ? 0 : pos;
-        pos = pos < a.max_seq - 1 ? pos : a.max_seq - 1;
-        const int tpos = pos < a.table_len - 1 ? pos : a.table_len - 1;
-        const long long kv_row =
-            (static_cast<long long>(sq) * a.n_kv * a.max_seq + pos) * static_cast<long long>(a.hd);
-        const uint32_t acc = tmem + lane_base + buf * C::ACC_STRIDE;
-        if (a.hd == 128) {
-#pragma unroll 1
-          for (int h = 0; h < BN / 128; ++h) {
-            const int head = (n0 >> 7) + h;
-            rope_head_epilogue<128>(a, acc + h * 128, head, tpos, kv_row, row,
-                                    valid && head * 128 < a.out_f);
-          }
-        } else {
-#pragma unroll 1
-          for (int h = 0; h < BN / 64; ++h) {
-            const int head = (n0 >> 6) + h;
-            rope_head_epilogue<64>(a, acc + h * 64, head, tpos, kv_row, row,
-                                   valid && head * 64 < a.out_f);
-          }
-        }
-        tc_fence_before_sync();
-        mbar_arrive(bar(ACC_EMPTY + buf));
-        continue;
-      }
       float *yrow = a.y + static_cast<long long>(row) * a.out_f;
 #pragma unroll 1
       for (int c0 = 0; c0 < BN; c0 += 32) {
@@ -551,7 +434,7 @@ wst_status_t operand_map(CUtensorMap *out, const void *base, int in_f, int rows,
   return WST_OK;
 }
 
-template <int BN, int KS, int RB, bool ROPE = false, bool INT4 = false>
+template <int BN, int KS, int RB, bool INT4 = false>
 wst_status_t launch_gemm(const void *w, const void *x, GemmArgs a, int sm_count) {
   using C = GCfg<BN, KS, RB>;
   CUtensorMap xmap, wmap;
@@ -567,7 +450,7 @@ wst_status_t launch_gemm(const void *w, const void *x, GemmArgs a, int sm_count)
   int dev = 0;
   WST_CUDA(cudaGetDevice(&dev));
   if (configured_dev != dev) {
-    WST_CUDA(cudaFuncSetAttribute(gemm_f16_kernel<BN, KS, RB, ROPE, INT4>,
+    WST_CUDA(cudaFuncSetAttribute(gemm_f16_kernel<BN, KS, RB, INT4>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
     configured_dev = dev;
   }
@@ -584,7 +467,7 @@ wst_status_t launch_gemm(const void *w, const void *x, GemmArgs a, int sm_count)
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_f16_kernel<BN, KS, RB, ROPE, INT4>, xmap, wmap, a);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_f16_kernel<BN, KS, RB, INT4>, xmap, wmap, a);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail("wst_gemm_fp16 (launch)", e);
   return WST_OK;
@@ -627,6 +510,18 @@ extern "C" wst_status_t wst_gemm_fp16(const void *w, const void *x, const void *
     return WST_OK;
   }
 
+  if (n > 128) {
+    PairGemm g;
+    g.w = w;
+    g.x = x;
+    g.bias = static_cast<const __half *>(bias);
+    g.y = static_cast<float *>(y);
+    g.in_f = in_f;
+    g.out_f = out_f;
+    g.n = n;
+    g.accum = accum;
+    return launch_gemm_pair(g, facts.sm_count);
+  }
   unsigned int *err_word = device_error_word();
   if (!err_word) return WST_ERR_CUDA;
   GemmArgs a{};
@@ -640,18 +535,14 @@ extern "C" wst_status_t wst_gemm_fp16(const void *w, const void *x, const void *
 
   /* Few tokens: the launch streams the weights once and is bound by how many SMs pull on
    * HBM, so the feature tile is the one of 32, 48 or 64 rows that gives a CTA the least
-   * to stream (6144 features: 128 tiles of 48; 4096: 128 tiles of 32).  Else 256-feature
-   * tiles for the tensor pipe. */
-  int bn = 256;
-  if (n <= 128) {
-    long long best = -1;
-    for (int cand : {64, 48, 32}) {
-      const long long tiles = (out_f + cand - 1) / cand;
-      const long long per_cta = (tiles + facts.sm_count - 1) / facts.sm_count * cand;
-      if (best < 0 || per_cta < best) { best = per_cta; bn = cand; }
-    }
+   * to stream (6144 features: 128 tiles of 48; 4096: 128 tiles of 32). */
+  int bn = 64;
+  long long best = -1;
+  for (int cand : {64, 48, 32}) {
+    const long long tiles = (out_f + cand - 1) / cand;
+    const long long per_cta = (tiles + facts.sm_count - 1) / facts.sm_count * cand;
+    if (best < 0 || per_cta < best) { best = per_cta; bn = cand; }
   }
-  if (n > 128) return launch_gemm<256, 1, 128>(w, x, a, facts.sm_count);
   /* a handful of tokens (decode-side chunks, speculative verification): four slabs of K
    * per request, and only the token rows that exist are fetched */
   if (in_f % 64 == 0 && n <= 16) return launch_narrow<4, 16>(bn, w, x, a, facts.sm_count);
@@ -677,6 +568,21 @@ extern "C" wst_status_t wst_gemm_int4_hier(const void *qw, const void *si, const
     return fail(WST_ERR_UNSUPPORTED_ARCH, "wst_gemm_int4_hier: this library is built for sm_100a only");
   if (n <= kInt4FewTokens)
     return launch_gemm_int4_few(qw, si, sb, x, bias, y, in_f, out_f, n, accum, facts.sm_count);
+  if (n > 128) {
+    PairGemm g;
+    g.name = "wst_gemm_int4_hier";
+    g.qw = static_cast<const uint4 *>(qw);
+    g.si = static_cast<const uint8_t *>(si);
+    g.sb = static_cast<const __half2 *>(sb);
+    g.x = x;
+    g.bias = static_cast<const __half *>(bias);
+    g.y = static_cast<float *>(y);
+    g.in_f = in_f;
+    g.out_f = out_f;
+    g.n = n;
+    g.accum = accum;
+    return launch_gemm_pair(g, facts.sm_count);
+  }
   unsigned int *err_word = device_error_word();
   if (!err_word) return WST_ERR_CUDA;
   GemmArgs a{};
@@ -690,10 +596,7 @@ extern "C" wst_status_t wst_gemm_int4_hier(const void *qw, const void *si, const
   a.qw = static_cast<const uint4 *>(qw);
   a.si = static_cast<const uint8_t *>(si);
   a.sb = static_cast<const __half2 *>(sb);
-  /* the token count decides the feature tile as for fp16 weights: 256 rows for the tensor
-   * pipe, 64 when the launch is a stream of the (four times smaller) weights */
-  if (n > 128) return launch_gemm<256, 1, 128, false, true>(nullptr, x, a, facts.sm_count);
-  return launch_gemm<64, 1, 128, false, true>(nullptr, x, a, facts.sm_count);
+  return launch_gemm<64, 1, 128, true>(nullptr, x, a, facts.sm_count);
 }
 
 static wst_status_t qkv_rope_append_common(
@@ -727,36 +630,35 @@ static wst_status_t qkv_rope_append_common(
   if (!device_facts(&facts)) return WST_ERR_CUDA;
   if (facts.cc_major < 10)
     return fail(WST_ERR_UNSUPPORTED_ARCH, "%s: this library is built for sm_100a only", name);
-  unsigned int *err_word = device_error_word();
-  if (!err_word) return WST_ERR_CUDA;
-  GemmArgs a{};
-  a.bias = static_cast<const __half *>(bias);
-  a.in_f = in_f;
-  a.out_f = static_cast<int>(out_f);
-  a.n = static_cast<int>(tokens);
-  a.err_word = err_word;
-  a.q_out = static_cast<__half *>(q_out);
-  a.k_cache = static_cast<__half *>(k_cache);
-  a.v_cache = static_cast<__half *>(v_cache);
-  a.cos_tab = static_cast<const float *>(cos_tab);
-  a.sin_tab = static_cast<const float *>(sin_tab);
-  a.q_gain = static_cast<const __half *>(q_norm_w);
-  a.k_gain = static_cast<const __half *>(k_norm_w);
-  a.seq_pos0 = static_cast<const int32_t *>(seq_pos0);
-  a.n_q = n_q;
-  a.n_kv = n_kv;
-  a.hd = head_dim;
-  a.n_per_seq = n;
-  a.max_seq = max_seq;
-  a.table_len = table_len;
-  a.eps = eps;
+  PairGemm g;
+  g.name = name;
+  g.w = w;
   if (qw) {
-    a.qw = static_cast<const uint4 *>(qw);
-    a.si = static_cast<const uint8_t *>(si);
-    a.sb = static_cast<const __half2 *>(sb);
-    return launch_gemm<256, 1, 128, true, true>(nullptr, x, a, facts.sm_count);
+    g.qw = static_cast<const uint4 *>(qw);
+    g.si = static_cast<const uint8_t *>(si);
+    g.sb = static_cast<const __half2 *>(sb);
   }
-  return launch_gemm<256, 1, 128, true>(w, x, a, facts.sm_count);
+  g.x = x;
+  g.bias = static_cast<const __half *>(bias);
+  g.in_f = in_f;
+  g.out_f = static_cast<int>(out_f);
+  g.n = static_cast<int>(tokens);
+  g.q_out = static_cast<__half *>(q_out);
+  g.k_cache = static_cast<__half *>(k_cache);
+  g.v_cache = static_cast<__half *>(v_cache);
+  g.cos_tab = static_cast<const float *>(cos_tab);
+  g.sin_tab = static_cast<const float *>(sin_tab);
+  g.q_gain = static_cast<const __half *>(q_norm_w);
+  g.k_gain = static_cast<const __half *>(k_norm_w);
+  g.seq_pos0 = static_cast<const int32_t *>(seq_pos0);
+  g.n_q = n_q;
+  g.n_kv = n_kv;
+  g.hd = head_dim;
+  g.n_per_seq = n;
+  g.max_seq = max_seq;
+  g.table_len = table_len;
+  g.eps = eps;
+  return launch_gemm_pair(g, facts.sm_count);
 }
 
 extern "C" wst_status_t wst_b200_qkv_rope_append_batch(

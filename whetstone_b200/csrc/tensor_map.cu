@@ -34,7 +34,7 @@ EncodeFn encoder() {
 
 wst_status_t make_kv_tensor_map(CUtensorMap *out, const void *base, int rank,
                                 const uint64_t *dims, const uint64_t *strides_bytes,
-                                const uint32_t *box) {
+                                const uint32_t *box, bool swizzled) {
   EncodeFn fn = encoder();
   if (!fn) return fail(WST_ERR_UNSUPPORTED_ARCH, "cuTensorMapEncodeTiled is not available");
   cuuint64_t d[5];
@@ -48,7 +48,7 @@ wst_status_t make_kv_tensor_map(CUtensorMap *out, const void *base, int rank,
   }
   CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, static_cast<cuuint32_t>(rank),
                   const_cast<void *>(base), d, s, b, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  swizzled ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS)
     return fail(WST_ERR_CUDA, "cuTensorMapEncodeTiled failed with CUresult %d", static_cast<int>(r));
@@ -72,7 +72,12 @@ wst_status_t cached_kv_tensor_map(CUtensorMap *out, const KvMapKey &key) {
     return WST_OK;
   }
   wst_status_t st;
-  if (key.rank == 5) {
+  if (key.rank == 2) {
+    uint64_t dims[3] = {key.d0, key.d1, 1};
+    uint64_t strides[2] = {key.d0 * 2, key.d0 * key.d1 * 2};
+    uint32_t box[3] = {32, key.b1, 1};
+    st = make_kv_tensor_map(out, key.base, 3, dims, strides, box, /*swizzled=*/false);
+  } else if (key.rank == 5) {
     /* page pool [pages][n_kv][16][128] seen as (64 columns, 16 rows, 2 column halves,
      * n_kv, pages): one box is both 128-byte halves of a page's 16 rows of one KV head,
      * 4 KB per request, laid down as [half][16 rows][128 B] */
