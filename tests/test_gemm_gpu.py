@@ -205,3 +205,15 @@ def test_more_than_128_tokens_at_the_edges_of_the_tiles(in_f, out_f, n):
     y0 = rng.standard_normal((n, out_f)).astype(np.float32)
     close(run(w, x, b, y0, True), orc.gemm_fp16(w, x, b, y0), 2e-4, f"{in_f} x {out_f} x {n}, accumulating")
     close(run(w, x, None, None, False), orc.gemm_fp16(w, x), 2e-4, f"{in_f} x {out_f} x {n}")
+
+
+@pytest.mark.parametrize("n", [64, 65, 80, 81, 96, 97, 128])
+@pytest.mark.parametrize("in_f,out_f", [(640, 4100), (320, 7000), (192, 12000)])   # 32, 48, 64 features a tile
+def test_up_to_128_tokens_at_the_edges_of_the_row_choices(in_f, out_f, n):
+    """Token rows fetched per tile (64, 80, 96, 128) either side of their edges with each
+    feature tile; in_f 320 and 192 end inside a request of several slabs."""
+    rng = np.random.default_rng(n + in_f)
+    w = (rng.standard_normal((out_f, in_f)) / np.sqrt(in_f)).astype(np.float16)
+    x = rng.standard_normal((n, in_f)).astype(np.float16)
+    y0 = rng.standard_normal((n, out_f)).astype(np.float32)
+    close(run(w, x, None, y0, True), orc.gemm_fp16(w, x, None, y0), 2e-4, f"{in_f} x {out_f} x {n}")

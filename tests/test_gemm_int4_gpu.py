@@ -167,3 +167,19 @@ def test_more_than_128_tokens_at_the_edges_of_the_tiles(in_f, out_f, n):
     got, _ = run(qw, si, sb, x, b, y0, in_f, out_f, True)
     close(got, orc.gemm_int4_hier(qw, si, sb, x, in_f, out_f, b, y0),
           3e-3 * max(1.0, (in_f / 896) ** 0.5), f"{in_f} x {out_f} x {n}")
+
+
+# K cut evenly, unevenly, with CTAs left without any (9 stages over 8), one stage; rows per CTA 64 and 128
+@pytest.mark.parametrize("in_f,out_f", [(3584, 2400), (1120, 330), (1056, 70), (128, 9000), (32, 17)])
+@pytest.mark.parametrize("n", [17, 33, 64, 65, 113, 128])
+def test_17_to_128_tokens_at_the_edges_of_the_tiles(in_f, out_f, n):
+    """The kernel whose clusters split K: token counts either side of the MMA's steps of 16,
+    rows cut off, scale bytes with and without four-byte alignment."""
+    qw, si, sb = fast_packed_weights(in_f, out_f, in_f + out_f + n)
+    rng = np.random.default_rng(n + in_f)
+    x = rng.uniform(-1, 1, (n, in_f)).astype(np.float16)
+    b = rng.standard_normal(out_f).astype(np.float16)
+    y0 = rng.standard_normal((n, out_f)).astype(np.float32)
+    got, _ = run(qw, si, sb, x, b, y0, in_f, out_f, True)
+    close(got, orc.gemm_int4_hier(qw, si, sb, x, in_f, out_f, b, y0),
+          3e-3 * max(1.0, (in_f / 896) ** 0.5), f"{in_f} x {out_f} x {n}")

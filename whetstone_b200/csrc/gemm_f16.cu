@@ -59,7 +59,7 @@ struct GCfg {
   static constexpr int TMEM_COLS = 2 * ACC_STRIDE;
   static_assert(RB % 8 == 0 && NSTAGE >= 2, "stage geometry");
   /* the M = 128 read of the last slab of the last stage stays inside the ring */
-  static_assert(KS == 1 ? RB == 128 : 128 * 128 <= A_SLAB + B_BYTES, "over-read leaves the ring");
+  static_assert(RB == 128 || 128 * 128 <= A_SLAB + B_BYTES, "over-read leaves the ring");
 };
 
 struct GemmArgs {
@@ -68,20 +68,12 @@ struct GemmArgs {
   int in_f, out_f, n, accum;
   int m_tiles, n_tiles;
   unsigned int *err_word;
-  /* the int4 form (INT4): the weights come packed, one 16-byte word of 32 nibbles and one
-   * byte of two 4-bit scale indices per group of 32 along K, one (d, dmin) pair per row */
-  const uint4 *qw;       /* [out_f][in_f / 32] */
-  const uint8_t *si;     /* [out_f][in_f / 32]: ls | lm << 4 */
-  const __half2 *sb;     /* [out_f]: (d, dmin) */
 };
 
-/* Threads of a CTA: 4 epilogue warps, the MMA warp, the TMA warp, and for the int4 form
- * sixteen warps that unpack the weight tile into shared memory. */
-constexpr int kUnpackThreads = 512;
-constexpr int gemm_threads(bool int4) { return int4 ? 192 + kUnpackThreads : 192; }
+constexpr int kGemmThreads = 192; /* 4 epilogue warps, the MMA warp, the TMA warp */
 
-template <int BN, int KS, int RB, bool INT4>
-__global__ void __launch_bounds__(gemm_threads(INT4), 1)
+template <int BN, int KS, int RB>
+__global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_f16_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap,
                 const GemmArgs a) {
   using C = GCfg<BN, KS, RB>;
@@ -98,7 +90,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant_
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < NSTAGE; ++i) {
-      mbar_init(bar(FULL + i), INT4 ? 1 + kUnpackThreads / 32 : 1); /* the TMA lane (+ the unpacking warps) */
+      mbar_init(bar(FULL + i), 1);
       mbar_init(bar(EMPTY + i), 1);
     }
     for (int i = 0; i < 2; ++i) {
@@ -107,7 +99,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant_
     }
     mbar_init_fence();
     tma_prefetch_desc(&xmap);
-    if constexpr (!INT4) tma_prefetch_desc(&wmap);
+    tma_prefetch_desc(&wmap);
   }
   if (warp == 4) {
     tmem_alloc(smem_u32(tmem_slot), C::TMEM_COLS);
@@ -138,10 +130,8 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant_
             ok = false;
             break;
           }
-          mbar_arrive_expect_tx(bar(FULL + st), INT4 ? C::A_BYTES : C::STAGE_BYTES);
-          if constexpr (INT4) { /* the weight tile comes from the unpacking warps */
-            tma_load_3d(sbase + st * C::STAGE_BYTES, &xmap, bar(FULL + st), kb * C::BK, m0, 0);
-          } else if constexpr (KS == 1) { /* maps over [rows][in_f]: columns past in_f read as zero */
+          mbar_arrive_expect_tx(bar(FULL + st), C::STAGE_BYTES);
+          if constexpr (KS == 1) { /* maps over [rows][in_f]: columns past in_f read as zero */
             tma_load_3d(sbase + st * C::STAGE_BYTES, &xmap, bar(FULL + st), kb * C::BK, m0, 0);
             tma_load_3d(sbase + st * C::STAGE_BYTES + C::A_BYTES, &wmap, bar(FULL + st), kb * C::BK,
                         n0, 0);
@@ -149,131 +139,6 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant_
             tma_load_3d(sbase + st * C::STAGE_BYTES, &xmap, bar(FULL + st), 0, m0, kb * KS);
             tma_load_3d(sbase + st * C::STAGE_BYTES + C::A_BYTES, &wmap, bar(FULL + st), 0, n0,
                         kb * KS);
-          }
-        }
-      }
-    }
-  } else if (warp >= 6) {
-    /* ---------------------- int4 weights -> fp16 tile in the operand layout
-     * (cuda/hier.cuh:8-13, the arithmetic of cuda/chunk_gemm.cu:121-132).  A thread takes
-     * the groups g = tid, tid + 512, ... of the stage: row g / 2 of the tile, 32-column
-     * half g % 2 of the 64-column k-block = four 16-byte chunks of the row's 128 swizzled
-     * bytes. */
-    if constexpr (INT4) {
-      /* The packed words of a group are one dependent load from DRAM; a thread that asked
-       * for them only when their stage fell free spent a memory latency per k-block (228 us
-       * for the projection that takes 101 with fp16 weights).  So each thread keeps the
-       * words of its groups for the next kAhead k-blocks in registers. */
-      constexpr int kAhead = 4;
-      constexpr int G = 2 * BN / kUnpackThreads > 0 ? 2 * BN / kUnpackThreads : 1;
-      const int tid = threadIdx.x - 6 * 32;
-      const int vec_per_row = a.in_f / 32;
-      const int my_tiles = blockIdx.x < n_tiles_total
-                               ? (n_tiles_total - 1 - static_cast<int>(blockIdx.x)) / static_cast<int>(gridDim.x) + 1
-                               : 0;
-      const int total = my_tiles * k_blocks;
-      struct Raw { /* as loaded: nothing may depend on these before their stage is unpacked */
-        uint4 w;
-        unsigned idx;
-        __half2 dd;
-      };
-      Raw ahead[kAhead][G];
-      /* the fetch cursor walks (tile, k-block) in the order of the stages; everything that
-       * needs a division is recomputed once per tile (the unpacking warps are bound by the
-       * instructions they issue: with the tile and k-block derived from the stage counter
-       * by three divisions per k-block, the address arithmetic cost as much as the
-       * unpacking) */
-      int f_left = total, f_kb = 0, f_tile = blockIdx.x;
-      size_t f_at[G];   /* group index of (row, half) at k-block 0 of the cursor's tile */
-      bool f_row_ok[G];
-      int f_grow[G];
-      auto fetch_tile = [&]() {
-        const int n0 = (f_tile / a.m_tiles) * BN;
-#pragma unroll
-        for (int j = 0; j < G; ++j) {
-          const int g = tid + j * kUnpackThreads;
-          const int grow = n0 + (g >> 1);
-          f_row_ok[j] = g < 2 * BN && grow < a.out_f;
-          f_grow[j] = grow;
-          f_at[j] = static_cast<size_t>(grow) * vec_per_row + (g & 1);
-        }
-      };
-      fetch_tile();
-      auto fetch = [&](Raw (&dst)[G]) {
-#pragma unroll
-        for (int j = 0; j < G; ++j) {
-          dst[j].w = make_uint4(0u, 0u, 0u, 0u);
-          dst[j].idx = 0u;
-          dst[j].dd = __float2half2_rn(0.f); /* past the last row or the last group: zeros */
-          const int v = f_kb * 2 + ((tid + j * kUnpackThreads) & 1);
-          if (f_left > 0 && f_row_ok[j] && v < vec_per_row) {
-            const size_t at = f_at[j] + 2 * f_kb;
-            dst[j].w = __ldg(a.qw + at);
-            dst[j].idx = __ldg(a.si + at);
-            dst[j].dd = __ldg(a.sb + f_grow[j]);
-          }
-        }
-        --f_left;
-        if (++f_kb == k_blocks) {
-          f_kb = 0;
-          f_tile += gridDim.x;
-          if (f_left > 0) fetch_tile();
-        }
-      };
-      auto unpack = [&](int it, const Raw (&src)[G]) -> bool {
-        const int st = it % NSTAGE;
-        if (it >= NSTAGE && !mbar_wait(bar(EMPTY + st), ((it / NSTAGE) - 1) & 1, a.err_word, 0x605u))
-          return false;
-        uint8_t *btile = smem + st * C::STAGE_BYTES + C::A_BYTES;
-#pragma unroll
-        for (int j = 0; j < G; ++j) {
-          const int g = tid + j * kUnpackThreads;
-          if (g < 2 * BN) {
-            const int row = g >> 1, half = g & 1;
-            const uint32_t words[4] = {src[j].w.x, src[j].w.y, src[j].w.z, src[j].w.w};
-            /* A nibble q dropped into byte 2 of 0x3F000000 is the float 0.5 + q / 256, one
-             * byte permute per weight; then w = q s - dmin lm = (256 s) f - (128 s + dmin lm)
-             * with s = d * ls is ONE fp32 fma per weight, and the result is rounded to fp16
-             * once -- the only difference from the exact weight, random in sign.  (In half2
-             * arithmetic, (q * ls) * d - fp16(lm * dmin), the rounded offset is common to the
-             * 32 weights of a group and adds up along the group: 9.7e-3 from the exact
-             * product on the engine's test case where this form has 1.3e-3 and the engine's
-             * own kernel 7.7e-3, for 6 % less time.) */
-            const float2 dd = __half22float2(src[j].dd);
-            const float s1 = dd.x * static_cast<float>(src[j].idx & 0xFu); /* d * ls */
-            const float sc = 256.0f * s1;
-            const float mt = fmaf(-128.0f, s1, -dd.y * static_cast<float>(src[j].idx >> 4));
-#pragma unroll
-            for (int wi = 0; wi < 4; ++wi) { /* 8 weights = one 16-byte chunk per word */
-              const uint32_t even = words[wi] & 0x0F0F0F0Fu, odd = (words[wi] >> 4) & 0x0F0F0F0Fu;
-              uint32_t o[4];
-#pragma unroll
-              for (int i = 0; i < 4; ++i) { /* weights 2i (low nibble of byte i) and 2i + 1 */
-                const float f0 = __uint_as_float(__byte_perm(even, 0x3F000000u, 0x7044u | (i << 8)));
-                const float f1 = __uint_as_float(__byte_perm(odd, 0x3F000000u, 0x7044u | (i << 8)));
-                o[i] = pack_half2(fmaf(f0, sc, mt), fmaf(f1, sc, mt));
-              }
-              *reinterpret_cast<uint4 *>(btile + swz128(row, half * 4 + wi)) =
-                  make_uint4(o[0], o[1], o[2], o[3]);
-            }
-          }
-        }
-        /* one arrival per warp: 256 arrivals on one barrier word took longer than the
-         * unpacking itself */
-        fence_async_smem();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar(FULL + st));
-        return true;
-      };
-#pragma unroll
-      for (int u = 0; u < kAhead; ++u) fetch(ahead[u]);
-      bool ok = true;
-      for (int it0 = 0; ok && it0 < total; it0 += kAhead) {
-#pragma unroll
-        for (int u = 0; u < kAhead; ++u) {
-          if (it0 + u < total) {
-            ok = ok && unpack(it0 + u, ahead[u]);
-            fetch(ahead[u]);
           }
         }
       }
@@ -434,23 +299,19 @@ wst_status_t operand_map(CUtensorMap *out, const void *base, int in_f, int rows,
   return WST_OK;
 }
 
-template <int BN, int KS, int RB, bool INT4 = false>
+template <int BN, int KS, int RB>
 wst_status_t launch_gemm(const void *w, const void *x, GemmArgs a, int sm_count) {
   using C = GCfg<BN, KS, RB>;
   CUtensorMap xmap, wmap;
   wst_status_t st = operand_map(&xmap, x, a.in_f, a.n, RB, KS);
   if (st != WST_OK) return st;
-  if (INT4) {
-    wmap = xmap; /* not used: the weight tile is unpacked by the CTA itself */
-  } else {
-    st = operand_map(&wmap, w, a.in_f, a.out_f, BN, KS);
-    if (st != WST_OK) return st;
-  }
+  st = operand_map(&wmap, w, a.in_f, a.out_f, BN, KS);
+  if (st != WST_OK) return st;
   static thread_local int configured_dev = -1;
   int dev = 0;
   WST_CUDA(cudaGetDevice(&dev));
   if (configured_dev != dev) {
-    WST_CUDA(cudaFuncSetAttribute(gemm_f16_kernel<BN, KS, RB, INT4>,
+    WST_CUDA(cudaFuncSetAttribute(gemm_f16_kernel<BN, KS, RB>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
     configured_dev = dev;
   }
@@ -459,7 +320,7 @@ wst_status_t launch_gemm(const void *w, const void *x, GemmArgs a, int sm_count)
   const long long tiles = static_cast<long long>(a.m_tiles) * a.n_tiles;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(static_cast<unsigned>(tiles < sm_count ? tiles : sm_count));
-  cfg.blockDim = dim3(gemm_threads(INT4));
+  cfg.blockDim = dim3(kGemmThreads);
   cfg.dynamicSmemBytes = C::SMEM_BYTES;
   cfg.stream = current_stream();
   cudaLaunchAttribute attr[1];
@@ -467,18 +328,36 @@ wst_status_t launch_gemm(const void *w, const void *x, GemmArgs a, int sm_count)
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_f16_kernel<BN, KS, RB, INT4>, xmap, wmap, a);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_f16_kernel<BN, KS, RB>, xmap, wmap, a);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail("wst_gemm_fp16 (launch)", e);
   return WST_OK;
 }
 
-template <int KS, int RB>
+/* Four slabs of K per request where three stages of them fit the ring, else two: with two
+ * stages a CTA waits for one request at a time (80 tokens of 3584 -> 4608, 32 features: 14.1 us
+ * with 128 token rows in two stages, 11.2 with 80 or 96 in three; 128 tokens: 14.7 us in two
+ * stages of four slabs, 12.6 in five of two). */
+template <int BN, int RB>
+constexpr int slabs_for() {
+  return 3 * 4 * (RB + BN) * 128 <= 200 * 1024 ? 4 : 2;
+}
+
+template <int RB>
 wst_status_t launch_narrow(int bn, const void *w, const void *x, const GemmArgs &a, int sm_count) {
   switch (bn) {
-    case 32: return launch_gemm<32, KS, RB>(w, x, a, sm_count);
-    case 48: return launch_gemm<48, KS, RB>(w, x, a, sm_count);
-    default: return launch_gemm<64, KS, RB>(w, x, a, sm_count);
+    case 32: return launch_gemm<32, slabs_for<32, RB>(), RB>(w, x, a, sm_count);
+    case 48: return launch_gemm<48, slabs_for<48, RB>(), RB>(w, x, a, sm_count);
+    default: return launch_gemm<64, slabs_for<64, RB>(), RB>(w, x, a, sm_count);
+  }
+}
+
+/* any in_f: one slab per request, from the matrix as it lies */
+wst_status_t launch_ragged(int bn, const void *w, const void *x, const GemmArgs &a, int sm_count) {
+  switch (bn) {
+    case 32: return launch_gemm<32, 1, 128>(w, x, a, sm_count);
+    case 48: return launch_gemm<48, 1, 128>(w, x, a, sm_count);
+    default: return launch_gemm<64, 1, 128>(w, x, a, sm_count);
   }
 }
 
@@ -543,12 +422,13 @@ extern "C" wst_status_t wst_gemm_fp16(const void *w, const void *x, const void *
     const long long per_cta = (tiles + facts.sm_count - 1) / facts.sm_count * cand;
     if (best < 0 || per_cta < best) { best = per_cta; bn = cand; }
   }
-  /* a handful of tokens (decode-side chunks, speculative verification): four slabs of K
-   * per request, and only the token rows that exist are fetched */
-  if (in_f % 64 == 0 && n <= 16) return launch_narrow<4, 16>(bn, w, x, a, facts.sm_count);
-  if (in_f % 64 == 0 && n <= 64) return launch_narrow<4, 64>(bn, w, x, a, facts.sm_count);
-  if (in_f % 64 == 0) return launch_narrow<4, 128>(bn, w, x, a, facts.sm_count);
-  return launch_narrow<1, 128>(bn, w, x, a, facts.sm_count);
+  if (in_f % 64 != 0) return launch_ragged(bn, w, x, a, facts.sm_count);
+  /* only about as many token rows as exist are fetched */
+  if (n <= 16) return launch_narrow<16>(bn, w, x, a, facts.sm_count);
+  if (n <= 64) return launch_narrow<64>(bn, w, x, a, facts.sm_count);
+  if (n <= 80) return launch_narrow<80>(bn, w, x, a, facts.sm_count);
+  if (n <= 96) return launch_narrow<96>(bn, w, x, a, facts.sm_count);
+  return launch_narrow<128>(bn, w, x, a, facts.sm_count);
 }
 
 extern "C" wst_status_t wst_gemm_int4_hier(const void *qw, const void *si, const void *sb,
@@ -566,37 +446,24 @@ extern "C" wst_status_t wst_gemm_int4_hier(const void *qw, const void *si, const
   if (!device_facts(&facts)) return WST_ERR_CUDA;
   if (facts.cc_major < 10)
     return fail(WST_ERR_UNSUPPORTED_ARCH, "wst_gemm_int4_hier: this library is built for sm_100a only");
-  if (n <= kInt4FewTokens)
+  /* A handful of tokens: unpacked in registers, every CTA with x to itself.  From 17 tokens on
+   * that costs 0.97 us per 2^20 weights where the kernel that shares x costs 0.48 and 3 us more
+   * per launch: 24 tokens of 896 -> 1152 take 3.6 and 5.7 us, of 3584 -> 4608 18 and 13. */
+  if (n <= 16 || (n <= kInt4FewTokens && static_cast<long long>(in_f) * out_f <= (6ll << 20)))
     return launch_gemm_int4_few(qw, si, sb, x, bias, y, in_f, out_f, n, accum, facts.sm_count);
-  if (n > 128) {
-    PairGemm g;
-    g.name = "wst_gemm_int4_hier";
-    g.qw = static_cast<const uint4 *>(qw);
-    g.si = static_cast<const uint8_t *>(si);
-    g.sb = static_cast<const __half2 *>(sb);
-    g.x = x;
-    g.bias = static_cast<const __half *>(bias);
-    g.y = static_cast<float *>(y);
-    g.in_f = in_f;
-    g.out_f = out_f;
-    g.n = n;
-    g.accum = accum;
-    return launch_gemm_pair(g, facts.sm_count);
-  }
-  unsigned int *err_word = device_error_word();
-  if (!err_word) return WST_ERR_CUDA;
-  GemmArgs a{};
-  a.bias = static_cast<const __half *>(bias);
-  a.y = static_cast<float *>(y);
-  a.in_f = in_f;
-  a.out_f = out_f;
-  a.n = n;
-  a.accum = accum;
-  a.err_word = err_word;
-  a.qw = static_cast<const uint4 *>(qw);
-  a.si = static_cast<const uint8_t *>(si);
-  a.sb = static_cast<const __half2 *>(sb);
-  return launch_gemm<64, 1, 128, true>(nullptr, x, a, facts.sm_count);
+  PairGemm g;
+  g.name = "wst_gemm_int4_hier";
+  g.qw = static_cast<const uint4 *>(qw);
+  g.si = static_cast<const uint8_t *>(si);
+  g.sb = static_cast<const __half2 *>(sb);
+  g.x = x;
+  g.bias = static_cast<const __half *>(bias);
+  g.y = static_cast<float *>(y);
+  g.in_f = in_f;
+  g.out_f = out_f;
+  g.n = n;
+  g.accum = accum;
+  return n > 128 ? launch_gemm_pair(g, facts.sm_count) : launch_gemm_narrow(g);
 }
 
 static wst_status_t qkv_rope_append_common(

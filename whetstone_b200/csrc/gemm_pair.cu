@@ -24,6 +24,7 @@
  * Products are exact in fp32 and accumulated in fp32. */
 
 #include "gemm_pair.cuh"
+#include "int4_tile.cuh"
 #include "tensor_map.cuh"
 #include "wst_ptx.cuh"
 
@@ -43,9 +44,8 @@ struct PairCfg {
   static constexpr int A_BYTES = KS * A_SLAB, B_BYTES = KS * B_SLAB;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int NSTAGE = (192 * 1024) / STAGE_BYTES;
-  /* packed words and scale bytes of one stage: 64 and 4 bytes per row */
-  static constexpr int PACK_BYTES = BH * 64;
-  static constexpr int SLOT_BYTES = BH * 68;
+  /* packed words and scale bytes of one stage */
+  static constexpr int SLOT_BYTES = slot_bytes(BH);
   static constexpr int NSLOT = !INT4 ? 0 : 26112 / SLOT_BYTES < 8 ? 26112 / SLOT_BYTES : 8;
   static constexpr int OFF_PACK = NSTAGE * STAGE_BYTES;
   static constexpr int EC = INT4 ? 16 : 32; /* columns that the epilogue stages at a time */
@@ -62,7 +62,7 @@ struct PairCfg {
   static constexpr int STAGE_WARPS = BH / (8 * UNITS);
   static constexpr int SETS = kUnpackWarps / STAGE_WARPS;
   static_assert(SMEM_BYTES <= 227 * 1024 && TMEM_COLS <= 512, "does not fit");
-  static_assert(PACK_BYTES + 4 * BH == SLOT_BYTES && SLOT_BYTES % 128 == 0 && SETS >= 1, "slot geometry");
+  static_assert(SLOT_BYTES % 128 == 0 && SETS >= 1, "slot geometry");
 };
 
 struct PairArgs {
@@ -73,14 +73,6 @@ struct PairArgs {
 
 /* ---- two-CTA forms of the tcgen05 and mbarrier instructions */
 
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
-}
 /* the same shared-memory offset in the pair's first CTA */
 __device__ __forceinline__ uint32_t in_leader(uint32_t addr) {
   uint32_t r;
@@ -131,17 +123,6 @@ __device__ __forceinline__ void pair_umma_commit(uint32_t bar) {
       ::"r"(bar), "h"(static_cast<uint16_t>(3))
       : "memory");
 }
-__device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-        "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr)
-      : "memory");
-}
-
 /* y += v on four floats, 16-byte aligned; no other thread adds to them */
 __device__ __forceinline__ void red_add_v4(float *y, float4 v) {
   asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(y), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
@@ -337,52 +318,25 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
   } else if (INT4 && warp == 6) {
     /* -------------------------------- packed words and scale bytes of this CTA's rows */
     if constexpr (INT4) {
-      const int groups = g.in_f / 32;
-      /* four scale bytes of a row and stage in one asynchronous copy where they lie aligned */
-      const bool quads = groups % 4 == 0 && (reinterpret_cast<uintptr_t>(g.si) & 3) == 0;
       int it = 0;
       bool ok = true;
       for (int tile = first_tile; ok && tile < n_tiles_total; tile += tile_step) {
-        const int n0 = (tile / a.m_tiles) * BN + rank * C::BH;
+        const PackedRows<C::BH> packed(&wmap, g.si, g.in_f / 32, g.out_f,
+                                       (tile / a.m_tiles) * BN + rank * C::BH, lane);
         for (int kb = 0; kb < k_blocks; ++kb, ++it) {
           const int sl = it % C::NSLOT;
           if (it >= C::NSLOT) {
             const bool free = mbar_wait(bar(P_EMPTY + sl), ((it / C::NSLOT) - 1) & 1, a.err_word, 0x707u);
             if (!__all_sync(0xffffffffu, free)) { ok = false; break; }
           }
-          const uint32_t slot = sbase + C::OFF_PACK + sl * C::SLOT_BYTES;
-          if (lane == 0) {
-            mbar_arrive_expect_tx(bar(P_FULL + sl), C::PACK_BYTES);
-            tma_load_3d(slot, &wmap, bar(P_FULL + sl), kb * (C::BK / 4), n0, 0);
-          }
-          for (int r = lane; r < C::BH; r += 32) {
-            const bool in = n0 + r < g.out_f;
-            const size_t at = static_cast<size_t>(in ? n0 + r : 0) * groups + 4 * kb;
-            const uint32_t dst = slot + C::PACK_BYTES + 4 * r;
-            if (quads) { /* past the last row: zeros */
-              asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(g.si + at),
-                           "r"(in ? 4 : 0)
-                           : "memory");
-            } else {
-              uint32_t v = 0;
-#pragma unroll
-              for (int j = 0; j < 4; ++j)
-                if (in && 4 * kb + j < groups) v |= static_cast<uint32_t>(__ldg(g.si + at + j)) << (8 * j);
-              asm volatile("st.shared.u32 [%0], %1;" ::"r"(dst), "r"(v) : "memory");
-            }
-          }
-          if (quads)
-            asm volatile("cp.async.mbarrier.arrive.noinc.shared.b64 [%0];" ::"r"(bar(P_FULL + sl)) : "memory");
-          else
-            mbar_arrive(bar(P_FULL + sl));
+          packed.fetch(sbase + C::OFF_PACK + sl * C::SLOT_BYTES, bar(P_FULL + sl), kb, lane);
         }
       }
-      if (quads) asm volatile("cp.async.wait_all;" ::: "memory");
+      fetch_packed_drain();
     }
   } else if (warp > 6) {
-    /* ---------------------- int4 weights -> this CTA's half of the fp16 tile, in the operand
-     * layout (cuda/hier.cuh:8-13, the arithmetic of cuda/chunk_gemm.cu:121-132).  A warp takes
-     * 8 rows x 4 groups of 32 weights = its rows' 128 columns of the stage. */
+    /* ---------------------- int4 weights -> this CTA's half of the fp16 tile.  A warp takes
+     * UNITS times 8 rows x 4 groups of 32 weights = its rows' 128 columns of the stage. */
     if constexpr (INT4) {
       const int uw = warp - 7;
       const int row0 = (uw % C::STAGE_WARPS) * 8 * C::UNITS + (lane >> 2), j = lane & 3;
@@ -408,41 +362,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
              (it < NSTAGE || mbar_wait(bar(EMPTY + st), ((it / NSTAGE) - 1) & 1, a.err_word, 0x705u));
         if (!__all_sync(0xffffffffu, ok)) break;
         const uint8_t *slot = smem + C::OFF_PACK + sl * C::SLOT_BYTES;
-        uint8_t *slab = smem + st * C::STAGE_BYTES + C::A_BYTES + (j >> 1) * C::B_SLAB;
-        /* the two slabs' lanes take their words in different order: the eight 16-byte stores
-         * of a phase, two rows x four groups, then fall on eight different bank groups */
-        const bool swap = j >= 2;
 #pragma unroll
-        for (int u = 0; u < C::UNITS; ++u) {
-          const int row = row0 + 8 * u;
-          /* columns past in_f came as zeros and meet zeros of x */
-          const uint4 w = *reinterpret_cast<const uint4 *>(slot + row * 64 + j * 16);
-          const unsigned idx = slot[C::PACK_BYTES + row * 4 + j];
-          /* A nibble q dropped into byte 2 of 0x3F000000 is the float 0.5 + q / 256, one byte
-           * permute per weight; then w = q s - dmin lm = (256 s) f - (128 s + dmin lm) with
-           * s = d * ls is ONE fp32 fma per weight, and the result is rounded to fp16 once -- the
-           * only difference from the exact weight, random in sign.  (In half2 arithmetic the
-           * rounded offset is common to the 32 weights of a group and adds up along it: 9.7e-3
-           * from the exact product on the engine's test case where this form has 1.3e-3.) */
-          const float s1 = dd[u].x * static_cast<float>(idx & 0xFu); /* d * ls */
-          const float sc = 256.0f * s1;
-          const float mt = fmaf(-128.0f, s1, -dd[u].y * static_cast<float>(idx >> 4));
-          const uint32_t words[4] = {swap ? w.z : w.x, swap ? w.w : w.y, swap ? w.x : w.z,
-                                     swap ? w.y : w.w};
-#pragma unroll
-          for (int wi = 0; wi < 4; ++wi) { /* 8 weights = one 16-byte chunk per word */
-            const uint32_t even = words[wi] & 0x0F0F0F0Fu, odd = (words[wi] >> 4) & 0x0F0F0F0Fu;
-            uint32_t o[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) { /* weights 2i (low nibble of byte i) and 2i + 1 */
-              const float f0 = __uint_as_float(__byte_perm(even, 0x3F000000u, 0x7044u | (i << 8)));
-              const float f1 = __uint_as_float(__byte_perm(odd, 0x3F000000u, 0x7044u | (i << 8)));
-              o[i] = pack_half2(fmaf(f0, sc, mt), fmaf(f1, sc, mt));
-            }
-            const int chunk = (j & 1) * 4 + (swap ? wi ^ 2 : wi);
-            *reinterpret_cast<uint4 *>(slab + swz128(row, chunk)) = make_uint4(o[0], o[1], o[2], o[3]);
-          }
-        }
+        for (int u = 0; u < C::UNITS; ++u)
+          unpack_group<C::BH>(slot, smem + st * C::STAGE_BYTES + C::A_BYTES, row0 + 8 * u, j, dd[u]);
         fence_async_smem();
         __syncwarp();
         if (lane == 0) {
@@ -601,31 +523,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
     tc_fence_after_sync();
     pair_tmem_dealloc(tmem, C::TMEM_COLS);
   }
-}
-
-wst_status_t rows_map(CUtensorMap *out, const void *base, int in_f, int rows, int box_rows) {
-  KvMapKey key{};
-  key.rank = 3;
-  key.base = base;
-  key.d0 = static_cast<uint64_t>(in_f);
-  key.d1 = static_cast<uint64_t>(rows);
-  key.d2 = 1;
-  key.d3 = 1;
-  key.b1 = static_cast<uint32_t>(box_rows);
-  return cached_kv_tensor_map(out, key);
-}
-
-/* the packed words of 128 columns of `box_rows` rows, unswizzled */
-wst_status_t packed_map(CUtensorMap *out, const void *base, int row_elems, int rows, int box_rows) {
-  KvMapKey key{};
-  key.rank = 2;
-  key.base = base;
-  key.d0 = static_cast<uint64_t>(row_elems);
-  key.d1 = static_cast<uint64_t>(rows);
-  key.d2 = 1;
-  key.d3 = 1;
-  key.b1 = static_cast<uint32_t>(box_rows);
-  return cached_kv_tensor_map(out, key);
 }
 
 template <int BN, bool ROPE, bool INT4>

@@ -38,4 +38,7 @@ struct PairGemm {
 
 wst_status_t launch_gemm_pair(const PairGemm &g, int sm_count);
 
+/* The plain form with int4 weights for up to 128 tokens (gemm_narrow.cu). */
+wst_status_t launch_gemm_narrow(const PairGemm &g);
+
 }  // namespace wst

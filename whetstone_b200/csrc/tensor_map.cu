@@ -99,4 +99,28 @@ wst_status_t cached_kv_tensor_map(CUtensorMap *out, const KvMapKey &key) {
   return WST_OK;
 }
 
+wst_status_t rows_map(CUtensorMap *out, const void *base, int in_f, int rows, int box_rows) {
+  KvMapKey key{};
+  key.rank = 3;
+  key.base = base;
+  key.d0 = static_cast<uint64_t>(in_f);
+  key.d1 = static_cast<uint64_t>(rows);
+  key.d2 = 1;
+  key.d3 = 1;
+  key.b1 = static_cast<uint32_t>(box_rows);
+  return cached_kv_tensor_map(out, key);
+}
+
+wst_status_t packed_map(CUtensorMap *out, const void *base, int row_elems, int rows, int box_rows) {
+  KvMapKey key{};
+  key.rank = 2;
+  key.base = base;
+  key.d0 = static_cast<uint64_t>(row_elems);
+  key.d1 = static_cast<uint64_t>(rows);
+  key.d2 = 1;
+  key.d3 = 1;
+  key.b1 = static_cast<uint32_t>(box_rows);
+  return cached_kv_tensor_map(out, key);
+}
+
 }  // namespace wst

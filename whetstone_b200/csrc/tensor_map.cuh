@@ -32,4 +32,10 @@ struct KvMapKey {
 };
 wst_status_t cached_kv_tensor_map(CUtensorMap *out, const KvMapKey &key);
 
+/* Operands of the projections: fp16 [rows][in_f], box 64 columns x box_rows, swizzled; and the
+ * packed words of int4 weights, [rows][row_elems] of two bytes, box of 128 columns' 64 bytes x
+ * box_rows, row after row. */
+wst_status_t rows_map(CUtensorMap *out, const void *base, int in_f, int rows, int box_rows);
+wst_status_t packed_map(CUtensorMap *out, const void *base, int row_elems, int rows, int box_rows);
+
 }  // namespace wst
