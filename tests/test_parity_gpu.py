@@ -277,6 +277,35 @@ def test_chunk_matches_oracle(chunk_kernel_choice, n_q, n_kv, hd, pos0, n):
                           f"chunk {n_q}/{n_kv}/{hd} pos0 {pos0} n {n}")
 
 
+# a cluster of one tile per slice takes caches of 65 to 512 rows; 513 is the first it leaves
+@pytest.mark.parametrize("max_seq", [65, 128, 300, 449, 512, 513])
+@pytest.mark.parametrize("n_q,n_kv,hd", [(14, 2, 64), (28, 4, 128), (32, 8, 128), (96, 2, 128)])
+def test_decode_in_a_short_cache(n_q, n_kv, hd, max_seq):
+    """Slices that add up within a cluster: an empty prefix, a cut-off tile, slices without a
+    live row, a full cache; 7, 4 and 48 query heads per KV head."""
+    rng = np.random.default_rng(max_seq + n_q)
+    cache = decode.KvCache(n_kv, n_q, hd, max_seq)
+    fill_bits(cache.k, NAN16)
+    fill_bits(cache.v, NAN16)
+    k, v = rand16(rng, (n_kv, max_seq, hd)), rand16(rng, (n_kv, max_seq, hd))
+    for seq in (1, 63, 64, 65, max_seq - 1, max_seq):
+        cache.k[:, :seq], cache.v[:, :seq] = dev(k[:, :seq]), dev(v[:, :seq])
+        q = workloads.f16_values(rng, (n_q, hd))
+        out = torch.zeros(n_q * hd, dtype=torch.float16, device="cuda")
+        decode.attn_decode(dev(q), cache, out, n_q, decode.DeviceCursor(seq - 1))
+        assert_close_per_head(host(out).astype(np.float64).reshape(n_q, hd),
+                              orc.decode_attention(q, k, v, seq), f"seq {seq} of {max_seq}")
+    assert decode.device_error() == 0
+
+
+# 16 query rows and the row after, prefixes at which the KV range starts to be cut (256, 512)
+@pytest.mark.parametrize("n_q,n_kv,hd,n", [(28, 4, 128, 2), (28, 4, 128, 3), (32, 8, 128, 4), (32, 8, 128, 5),
+                                           (14, 2, 64, 2), (14, 2, 64, 3), (14, 2, 64, 18), (28, 4, 128, 19)])
+@pytest.mark.parametrize("end", [20, 128, 256, 257, 512, 513, 1300])
+def test_few_rows_behind_a_prefix(n_q, n_kv, hd, n, end):
+    test_chunk_matches_oracle(0, n_q, n_kv, hd, end - n, n)
+
+
 @pytest.mark.parametrize("ramp", [0.0, 0.02, 0.3, -0.3])
 def test_chunk_with_scores_that_drift_along_the_sequence(chunk_kernel_choice, ramp):
     """Scores that grow (or fall) steadily along the cache: the running exponent

@@ -41,6 +41,7 @@ using namespace ptx;
 
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
+constexpr int kMaxCluster = 8; /* slices that can be one cluster */
 
 struct RowsArgs {
   const float *q;
@@ -65,6 +66,7 @@ struct RowsArgs {
   int via_scratch; /* a single slice still writes its row to scratch: the merge kernel
                     * follows (it carries the cross-GPU exchange) */
   float out_scale; /* fp8 cache: the values' scale, applied to the accumulated rows */
+  int clustered;   /* the slices of a unit are one cluster and add up among themselves */
 };
 
 /* KV8: the cache holds e4m3 bytes.  A stage is then the raw K and V tiles, [BN rows][HD
@@ -93,6 +95,9 @@ struct Cfg {
   static constexpr int smem_bytes(int stages) {
     return stages * STAGE_BYTES + PRIV_BYTES + Q_BYTES + (2 * NSTAGE + 2) * 8 + 64 + 1024;
   }
+  /* clustered: the CTA's merged rows [ROWS][HD+4] lie behind the dump */
+  static constexpr int PART_BYTES = ROWS * (HD + 4) * 4;
+  static constexpr int CLUSTER_STAGES = (DUMP_BYTES + PART_BYTES + STAGE_BYTES - 1) / STAGE_BYTES;
   static_assert(MIN_STAGES <= NSTAGE, "combine buffer must fit the ring");
   static_assert(smem_bytes(NSTAGE) <= 232448, "shared memory of one CTA");
 };
@@ -617,7 +622,27 @@ attn_rows_kernel(const __grid_constant__ CUtensorMap kmap,
   consumer_bar(C::CTHREADS);
 
   const int unit = (s * a.n_kv + kvh) * a.n_rowblk + rb;
-  const bool direct = ns == 1 && !a.via_scratch;
+  const bool direct = (ns == 1 || a.clustered) && !a.via_scratch;
+  /* one finished cell: columns 4 c4 .. + 3 of row r */
+  auto emit = [&](int r, int c4, const float4 &acc, float M, float den) {
+    const int head = kvh * a.gqa + r % a.gqa;
+    if (!a.partial_out) {
+      const int tok = tok_begin + tok0 + r / a.gqa;
+      const float inv = den > 0.f ? 1.f / den : 0.f;
+      store_half4(static_cast<__half *>(a.out) +
+                      (static_cast<long long>(tok) * a.n_q + head) * HD + 4 * c4,
+                  acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
+    } else { /* the caller's (m, l, acc) triple, natural-log m */
+      float *dst = static_cast<float *>(a.out) + static_cast<long long>(head) * (HD + 2);
+      if (c4 == 0) {
+        dst[0] = M * kLn2;
+        dst[1] = den;
+      }
+      reinterpret_cast<float2 *>(dst + 2 + 4 * c4)[0] = make_float2(acc.x, acc.y);
+      reinterpret_cast<float2 *>(dst + 2 + 4 * c4)[1] = make_float2(acc.z, acc.w);
+    }
+  };
+  float *part = dump + C::DUMP_BYTES / 4; /* clustered: this CTA's rows */
   for (int idx = ctid; idx < rows_valid * (HD / 4); idx += C::CTHREADS) {
     const int r = idx / (HD / 4), c4 = idx % (HD / 4);
     const float *cell = dump + (static_cast<size_t>(r / RPG) * 4 * RPG + r % RPG) * DR;
@@ -643,21 +668,12 @@ attn_rows_kernel(const __grid_constant__ CUtensorMap kmap,
     if constexpr (KV8) { /* the stored values times their scale are the values */
       acc.x *= a.out_scale; acc.y *= a.out_scale; acc.z *= a.out_scale; acc.w *= a.out_scale;
     }
-    const int head = kvh * a.gqa + r % a.gqa;
-    if (direct && !a.partial_out) {
-      const int tok = tok_begin + tok0 + r / a.gqa;
-      const float inv = den > 0.f ? 1.f / den : 0.f;
-      store_half4(static_cast<__half *>(a.out) +
-                      (static_cast<long long>(tok) * a.n_q + head) * HD + 4 * c4,
-                  acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
-    } else if (direct) { /* the caller's (m, l, acc) triple, natural-log m */
-      float *dst = static_cast<float *>(a.out) + static_cast<long long>(head) * (HD + 2);
-      if (c4 == 0) {
-        dst[0] = M * kLn2;
-        dst[1] = den;
-      }
-      reinterpret_cast<float2 *>(dst + 2 + 4 * c4)[0] = make_float2(acc.x, acc.y);
-      reinterpret_cast<float2 *>(dst + 2 + 4 * c4)[1] = make_float2(acc.z, acc.w);
+    if (a.clustered) {
+      float *dst = part + r * DR;
+      *reinterpret_cast<float4 *>(dst + 4 * c4) = acc;
+      if (c4 == 0) *reinterpret_cast<float2 *>(dst + HD) = make_float2(M, den);
+    } else if (direct) {
+      emit(r, c4, acc, M, den);
     } else { /* this slice's row for the merge kernel */
       float *dst = a.scratch +
                    ((static_cast<long long>(unit) * ns + split) * a.rows_cap + r) * DR;
@@ -665,6 +681,45 @@ attn_rows_kernel(const __grid_constant__ CUtensorMap kmap,
       if (c4 == 0) *reinterpret_cast<float2 *>(dst + HD) = make_float2(M, den);
     }
   }
+  if (!a.clustered) return;
+
+  /* ---- the cluster's slices, added up through distributed shared memory: CTA after CTA takes
+   * cells, each reads all the slices' copies in the same order */
+  cluster_sync();
+  const uint32_t part_u32 = smem_u32(part);
+  for (int idx = split * C::CTHREADS + ctid; idx < rows_valid * (HD / 4); idx += ns * C::CTHREADS) {
+    const int r = idx / (HD / 4), c4 = idx % (HD / 4);
+    float4 v[kMaxCluster];
+    float2 ml[kMaxCluster];
+#pragma unroll
+    for (int p = 0; p < kMaxCluster; ++p) { /* all loads in flight together */
+      if (p < ns) {
+        const uint32_t row = in_cta(part_u32 + r * (DR * 4), p);
+        v[p] = ld_cluster_f32x4(row + 16 * c4);
+        ml[p] = ld_cluster_f32x2(row + HD * 4);
+      } else {
+        v[p] = make_float4(0.f, 0.f, 0.f, 0.f);
+        ml[p] = make_float2(-INFINITY, 0.f);
+      }
+    }
+    float M = -INFINITY;
+#pragma unroll
+    for (int p = 0; p < kMaxCluster; ++p) M = fmaxf(M, ml[p].x);
+    const float m_use = M == -INFINITY ? 0.f : M;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    float den = 0.f;
+#pragma unroll
+    for (int p = 0; p < kMaxCluster; ++p) {
+      const float wgt = ex2(ml[p].x - m_use);
+      acc.x = fmaf(wgt, v[p].x, acc.x);
+      acc.y = fmaf(wgt, v[p].y, acc.y);
+      acc.z = fmaf(wgt, v[p].z, acc.z);
+      acc.w = fmaf(wgt, v[p].w, acc.w);
+      den = fmaf(wgt, ml[p].y, den);
+    }
+    emit(r, c4, acc, M, den);
+  }
+  cluster_sync(); /* nobody reads this CTA's rows any more */
 }
 
 /* ---------------------------------------------------------- slice merge */
@@ -1119,17 +1174,21 @@ inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 
  * while its predecessor in the stream drains; it orders itself with
  * griddepcontrol.wait. */
 template <typename Kern, typename... Args>
-cudaError_t launch_pdl(Kern kern, dim3 grid, dim3 block, size_t smem, Args... args) {
+cudaError_t launch_pdl(Kern kern, dim3 grid, dim3 block, size_t smem, int cluster, Args... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = current_stream();
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = static_cast<unsigned>(cluster);
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
   cudaError_t e = cudaLaunchKernelEx(&cfg, kern, args...);
   return e == cudaSuccess ? cudaGetLastError() : e;
 }
@@ -1150,11 +1209,12 @@ wst_status_t launch_cfg(const RowsLaunch &L, const RowsArgs &args, const CUtenso
   /* the ring depth in use sizes the block's shared memory: at half the ring two blocks
    * (of consecutive launches) share an SM */
   RowsArgs sized = args;
-  if (sized.nstage < C::MIN_STAGES) sized.nstage = C::MIN_STAGES;
+  const int least = sized.clustered ? C::CLUSTER_STAGES : C::MIN_STAGES;
+  if (sized.nstage < least) sized.nstage = least;
   if (sized.nstage > C::NSTAGE) sized.nstage = C::NSTAGE;
   if (sized.early_depth > sized.nstage) sized.early_depth = sized.nstage;
-  cudaError_t e = launch_pdl(kern, grid, dim3(C::THREADS), C::smem_bytes(sized.nstage), kmap, vmap,
-                             sized);
+  cudaError_t e = launch_pdl(kern, grid, dim3(C::THREADS), C::smem_bytes(sized.nstage),
+                             sized.clustered ? sized.n_splits : 1, kmap, vmap, sized);
   if (e != cudaSuccess)
     return fail(WST_ERR_CUDA, "%s (launch): %s (%s)", L.name, cudaGetErrorString(e),
                 cudaGetErrorName(e));
@@ -1297,6 +1357,15 @@ wst_status_t launch_rows(const RowsLaunch &L) {
   a.tpb = tpb;
   a.rows_cap = rows_cap;
   a.via_scratch = exchange ? 1 : 0;
+  /* A short cache: a tile per slice, and the slices of a KV head as one cluster that adds up
+   * among its CTAs instead of through scratch and a second kernel.  Per layer of decode, both
+   * launches, 100 to 500 rows in a cache of 512: 5.7 -> 5.5 us (14 heads over 2 of 64), 6.6 ->
+   * 5.9 (28 over 4 of 128), 6.8 -> 6.2 (32 over 8).  With two tiles per CTA (1024 rows) the two
+   * are level, and longer caches need more SMs than a cluster has.  (Not for triples: they are
+   * compared with those of the exchange, which keep their slices.) */
+  if (decode_shape && !exchange && !L.partial_out && splits > 1 &&
+      (L.max_len + kRowsTile - 1) / kRowsTile <= kMaxCluster && splits <= kMaxCluster)
+    a.clustered = 1;
   const int max_stages = kRowsRingBytes / (L.hd == 128 ? 32768 : 16384);
   a.nstage = max_stages;
   if (decode_shape) a.nstage = L.hd == 128 ? kDecodeStages : 2 * kDecodeStages;
@@ -1340,7 +1409,7 @@ wst_status_t launch_rows(const RowsLaunch &L) {
     st = L.paged ? launch_shape<64, true>(L, a, kmap, vmap, grid, rows)
                  : launch_shape<64, false>(L, a, kmap, vmap, grid, rows);
   }
-  if (st != WST_OK || (splits == 1 && !exchange)) return st;
+  if (st != WST_OK || a.clustered || (splits == 1 && !exchange)) return st;
 
   SplitMerge m;
   m.scratch = L.scratch;
@@ -1391,12 +1460,12 @@ wst_status_t launch_split_merge(const SplitMerge &S) {
   if ((S.slice_counts || (S.n_splits <= 16 && S.rows_cap >= 16)) && !S.partial_out && S.world <= 1) {
     /* few slices, many rows (ragged verify, a sliced chunk): a warp per row */
     const dim3 rgrid(static_cast<unsigned>((S.rows_cap + 7) / 8), static_cast<unsigned>(S.n_units));
-    e = S.hd == 128 ? launch_pdl(attn_merge_rows_kernel<128>, rgrid, dim3(256), 0, m)
-                    : launch_pdl(attn_merge_rows_kernel<64>, rgrid, dim3(256), 0, m);
+    e = S.hd == 128 ? launch_pdl(attn_merge_rows_kernel<128>, rgrid, dim3(256), 0, 1, m)
+                    : launch_pdl(attn_merge_rows_kernel<64>, rgrid, dim3(256), 0, 1, m);
   } else {
     const dim3 mgrid(static_cast<unsigned>(S.rows_cap), static_cast<unsigned>(S.n_units));
-    e = S.hd == 128 ? launch_pdl(attn_merge_kernel<128>, mgrid, dim3(128), 0, m)
-                    : launch_pdl(attn_merge_kernel<64>, mgrid, dim3(128), 0, m);
+    e = S.hd == 128 ? launch_pdl(attn_merge_kernel<128>, mgrid, dim3(128), 0, 1, m)
+                    : launch_pdl(attn_merge_kernel<64>, mgrid, dim3(128), 0, 1, m);
   }
   if (e != cudaSuccess)
     return fail(WST_ERR_CUDA, "%s (merge launch): %s (%s)", S.name, cudaGetErrorString(e),

@@ -61,20 +61,6 @@ __device__ __forceinline__ void tma_prefetch_3d(const CUtensorMap *map, int c0, 
                "r"(c0), "r"(c1), "r"(c2)
                : "memory");
 }
-__device__ __forceinline__ uint32_t in_cta(uint32_t addr, int rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-  return r;
-}
-__device__ __forceinline__ float4 ld_cluster_v4(uint32_t addr) {
-  float4 v;
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-               : "r"(addr)
-               : "memory");
-  return v;
-}
-
 template <int ROWS>
 __global__ void __launch_bounds__(NarrowCfg<ROWS>::THREADS, 1)
 gemm_narrow_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap,
@@ -251,7 +237,7 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_consta
       float4 part[kMaxCluster];
 #pragma unroll
       for (int p = 0; p < kMaxCluster; ++p)
-        if (p < csize) part[p] = ld_cluster_v4(from[p] + tok * (ROWS * 4));
+        if (p < csize) part[p] = ld_cluster_f32x4(from[p] + tok * (ROWS * 4));
       float4 o = part[0];
 #pragma unroll
       for (int p = 1; p < kMaxCluster; ++p)
