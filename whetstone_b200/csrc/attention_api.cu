@@ -61,14 +61,19 @@ void note_unsplit(const char *who, const char *why) {
                "wst_b200_reserve_chunk_workspace once outside any capture", who, why);
 }
 
-/* Slices of the KV range for a chunk launch of `tiles` (unit, query tile) pairs
- * against at most `len` positions: none when the tiles fill the GPU by themselves or
- * the prefix is short; else enough to fill it, in runs of at least two KV tiles. */
+/* Slices of the KV range for a chunk launch of `tiles` (unit, query tile) pairs against at
+ * most `len` positions: none when the tiles fill the GPU by themselves or the prefix is short;
+ * else enough to fill it, in runs of at least two KV tiles.  A few rows cost the merge little:
+ * for them down to one KV tile each, behind 256 rows already (append and attention, 28 heads
+ * over 4 of 128: 5 tokens behind 4099 rows 12.1 us with 33 slices, 13.9 with 16; behind 450
+ * rows 9.8 and 11.6 unsplit.  128 tokens behind 1000 rows: 22.4 in runs of two, 23.3 of one;
+ * 256 tokens behind none or 256: 17.1 unsplit, 19.6 split). */
 int chunk_slices(int sm_count, long long tiles, int len) {
-  if (tiles <= 0 || tiles * 2 > sm_count || len <= 512) return 1;
+  const bool few = tiles <= 8;
+  if (tiles <= 0 || tiles * 2 > sm_count || len <= (few ? 256 : 512)) return 1;
   long long s = sm_count / tiles;
-  const long long kv_tiles = (len + 127) / 128;
-  if (s > kv_tiles / 2) s = kv_tiles / 2;
+  const long long most = (len + 127) / 128 / (few ? 1 : 2);
+  if (s > most) s = most;
   if (s > kRowsMaxSplits) s = kRowsMaxSplits;
   return s < 2 ? 1 : static_cast<int>(s);
 }
@@ -518,20 +523,21 @@ extern "C" wst_status_t wst_attn_chunk(const void *qkv, const void *k_cache,
   const bool tc_ok = choice != 1 && rows_kernel_supports(n_q, n_kv, head_dim, k_cache, v_cache) &&
                      aligned16(qkv);
 
-  /* 128-row tcgen05 tiles when the chunk is large enough to fill the GPU with
-   * them (or the prefix is short enough that it does not matter); a few tokens
-   * against a long prefix go to the split-KV kernel instead. */
-  bool use_prefill = tc_ok && choice != 2 && prefill_kernel_supports(n_q, n_kv, head_dim, n);
+  /* 128-row tcgen05 tiles, cut along the prefix where they do not fill the GPU.  They are
+   * ahead even where most of their rows are empty: 2 tokens behind 4099 rows 10.8 us with the
+   * append against 14.3 with the mma.sync row-block kernel, 5 tokens 12.1 and 19.3 (28 heads
+   * over 4 of 128).  A single 16-row block streams better where the prefix is short (2 tokens
+   * behind 300 rows: 8.2 against 9.8) and at head_dim 64 (7.7 against 8.0). */
+  const bool one_block = n * (n_q / n_kv) <= 16;
+  const bool use_prefill = tc_ok && choice != 2 &&
+                     (choice == 3 || choice == 4 ? prefill_kernel_supports(n_q, n_kv, head_dim, n)
+                                                 : !one_block || (head_dim == 128 && pos0 + n > 512));
   int splits = 1;
   if (use_prefill && choice != 3 && choice != 4) {
     DeviceFacts facts;
     if (!device_facts(&facts)) return WST_ERR_CUDA;
-    const int gqa = n_q / n_kv;
-    splits = chunk_slices(facts.sm_count, (static_cast<long long>(n) * gqa + 127) / 128 * n_kv,
-                          pos0 + n);
-    /* at most one mma.sync row tile per KV head against a long prefix: the decode
-     * kernel's row-block form streams that better than a 128-row tcgen05 tile */
-    if (splits > 1 && n * gqa <= 16) use_prefill = false;
+    splits = chunk_slices(facts.sm_count,
+                          (static_cast<long long>(n) * (n_q / n_kv) + 127) / 128 * n_kv, pos0 + n);
   }
   if (use_prefill) {
     PrefillLaunch P;
@@ -601,11 +607,7 @@ static wst_status_t chunk_batch_common(const void *qkv, bool q16, const void *k_
   const long long q_stride =
       q16 ? static_cast<long long>(n_q) * head_dim : static_cast<long long>(n_q + 2 * n_kv) * head_dim;
   const int choice = g_kernel_choice.load();
-  bool use_prefill = choice != 2 && prefill_kernel_supports(n_q, n_kv, head_dim, n);
-  if (use_prefill && choice != 3 && choice != 4 && !q16) {
-    const int gqa = n_q / n_kv;
-    use_prefill = (static_cast<long long>(n) * gqa + 127) / 128 * n_kv * n_seq >= 32;
-  }
+  const bool use_prefill = choice != 2 && prefill_kernel_supports(n_q, n_kv, head_dim, n);
   if (q16 && !use_prefill)
     return fail(WST_ERR_SHAPE,
                 "wst_b200_attn_chunk_batch_q16: fp16 query rows are taken by the tensor-core "
