@@ -1938,10 +1938,12 @@ wst_status_t launch_prefill(const PrefillLaunch &P) {
    * The one-tile kernel takes what is left: launches that finish sooner with one
    * tile per CTA (few tiles), paged caches, ragged batches and the sliced form. */
   /* waves x measured time per KV tile: a CTA with two query tiles takes 1.5 times as
-   * long per KV tile as a CTA with one (1.86 against 1.24 us) */
+   * long per KV tile as a CTA with one (1.86 against 1.24 us).  Level counts, two waves against
+   * three, go to the pairs: 6 x 256 tokens, 28 heads over 4, two chunks with their appends 75 us
+   * and 94, 3 x 509 tokens behind 2500 rows, 32 heads over 8, 227 and 257. */
   const long long tiles = units * a.n_qtiles, pairs = units * ((a.n_qtiles + 1) / 2);
   const long long sm = facts.sm_count;
-  const bool pays = (pairs + sm - 1) / sm * 3 < (tiles + sm - 1) / sm * 2;
+  const bool pays = (pairs + sm - 1) / sm * 3 <= (tiles + sm - 1) / sm * 2;
   const bool pair = P.force_pair >= 0 && (P.force_pair > 0 || (a.n_qtiles >= 2 && pays)) &&
                     splits == 1 && !P.page_table && !P.cu_tokens;
   const unsigned gx = splits > 1 ? a.n_qtiles * splits : (pair ? (a.n_qtiles + 1) / 2 : a.n_qtiles);
