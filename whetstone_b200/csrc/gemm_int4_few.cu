@@ -5,13 +5,12 @@
  *
  * What bounds it: the packed weights are read once (8.8 MB for 3584 -> 4608: 1.4 us of
  * HBM), and unpacking them costs about three instructions per weight (the same again over
- * 148 SMs).  The tensor-memory kernel of gemm_f16.cu serves such a call with 72 CTAs that
- * walk 56 k-blocks one barrier round trip at a time, three quarters of its unpacking warps
- * without a group to unpack.  Here nothing goes through shared memory and nothing waits for
- * another warp before the last step:
+ * 148 SMs).  With operand tiles in shared memory a handful of tokens pay a barrier round trip
+ * per k-block for nothing: no token shares another's.  Here nothing goes through shared memory
+ * and nothing waits for another warp before the last step:
  *
- *   - a CTA owns 16 * MT weight rows, its eight warps take interleaved 128-column slabs of
- *     K, so every SM pulls on HBM at once and a warp walks three or four slabs;
+ *   - a CTA owns 16 * MT weight rows, its warps take interleaved 128-column slabs of K, so
+ *     every SM pulls on HBM at once and a warp walks two to four slabs;
  *   - the order of K inside a slab is free as long as both operands agree on it: lane t of
  *     a quad takes the slab's t-th group of 32 weights of its rows -- one 16-byte load, the
  *     quad's four loads one 64-byte run -- unpacks it in registers and feeds
@@ -19,10 +18,10 @@
  *     group's columns, 16 bytes per step pair straight from L2;
  *   - the packed words a CTA will need are prefetched towards L2 before the grid dependency
  *     resolves (a prefetch has no architectural effect, whatever the launch ahead writes).
- * Measured, 5 tokens, 3584 -> 4608 and 3584 -> 3584 in turn over 28 layers of weights: 12.0
- * us per launch, where the host call is most of it, against 38.4 us.
+ * Measured, a launch in a graph, 5 tokens of 3584 -> 4608: 6.1 us; operand tiles and
+ * tensor memory took 38.
  *
- * Per weight the arithmetic is that of gemm_f16.cu: w = q (d ls) - dmin lm in one fp32 fma,
+ * Per weight the arithmetic is that of int4_tile.cuh: w = q (d ls) - dmin lm in one fp32 fma,
  * rounded to fp16 once; products and sums fp32. */
 
 #include "gemm_int4_few.cuh"
@@ -32,9 +31,6 @@ namespace wst {
 namespace {
 
 using namespace ptx;
-
-constexpr int kFewWarps = 8;
-constexpr int kFewThreads = 32 * kFewWarps;
 
 struct FewArgs {
   const uint4 *qw;    /* [out_f][in_f / 32] words of 32 nibbles */
@@ -53,11 +49,12 @@ struct Slab {
   uint8_t idx[2 * MT];
 };
 
-template <int MT, int NT>
-__global__ void __launch_bounds__(kFewThreads, 2) gemm_int4_few_kernel(const FewArgs a) {
+/* WARPS on a CTA: sixteen on an SM in one or two CTAs */
+template <int MT, int NT, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS, 16 / WARPS) gemm_int4_few_kernel(const FewArgs a) {
   constexpr int R = 16 * MT, RI = 2 * MT;
   constexpr int LD = R + 4; /* a warp's stores fall into 32 different banks */
-  __shared__ float red[kFewWarps][8 * NT][LD];
+  __shared__ float red[WARPS][8 * NT][LD];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
   const int row0 = blockIdx.x * R;
@@ -71,7 +68,7 @@ __global__ void __launch_bounds__(kFewThreads, 2) gemm_int4_few_kernel(const Few
     const int r = row0 + 8 * i + g;
     row[i] = r < a.out_f ? r : a.out_f - 1;
   }
-  for (int s = warp; s < slabs; s += kFewWarps)
+  for (int s = warp; s < slabs; s += WARPS)
     if (t == 0)
 #pragma unroll
       for (int i = 0; i < RI; ++i)
@@ -148,12 +145,12 @@ __global__ void __launch_bounds__(kFewThreads, 2) gemm_int4_few_kernel(const Few
   uint4 xb[RING][NT];
   if (warp < slabs) fetch(warp, buf[0]);
 #pragma unroll
-  for (int p = 0; p < RING; ++p) fetch_x(warp + (p >> 2) * kFewWarps, p & 3, xb[p]);
-  for (int s = warp; s < slabs; s += 2 * kFewWarps) {
+  for (int p = 0; p < RING; ++p) fetch_x(warp + (p >> 2) * WARPS, p & 3, xb[p]);
+  for (int s = warp; s < slabs; s += 2 * WARPS) {
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      if (s + h * kFewWarps >= slabs) break;
-      fetch(s + (h + 1) * kFewWarps, buf[h ^ 1]);
+      if (s + h * WARPS >= slabs) break;
+      fetch(s + (h + 1) * WARPS, buf[h ^ 1]);
       const Slab<MT> &d = buf[h];
       float sc[RI], mn[RI];
 #pragma unroll
@@ -166,7 +163,7 @@ __global__ void __launch_bounds__(kFewThreads, 2) gemm_int4_few_kernel(const Few
       for (int wi = 0; wi < 4; ++wi) {
         const int p = 4 * h + wi, next = p + RING;
         multiply(d, sc, mn, wi, xb[p % RING]);
-        fetch_x(s + (next >> 2) * kFewWarps, next & 3, xb[p % RING]);
+        fetch_x(s + (next >> 2) * WARPS, next & 3, xb[p % RING]);
       }
     }
   }
@@ -179,29 +176,29 @@ __global__ void __launch_bounds__(kFewThreads, 2) gemm_int4_few_kernel(const Few
       for (int c = 0; c < 4; ++c)
         red[warp][8 * nt + 2 * t + (c & 1)][16 * mt + g + 8 * (c >> 1)] = acc[mt][nt][c];
   __syncthreads();
-  for (int i = threadIdx.x; i < 8 * NT * R; i += kFewThreads) {
+  for (int i = threadIdx.x; i < 8 * NT * R; i += 32 * WARPS) {
     const int tok = i / R, r = i % R;
     if (tok >= a.n || row0 + r >= a.out_f) continue;
     float sum = a.bias ? __half2float(a.bias[row0 + r]) : 0.f;
 #pragma unroll
-    for (int w = 0; w < kFewWarps; ++w) sum += red[w][tok][r];
+    for (int w = 0; w < WARPS; ++w) sum += red[w][tok][r];
     float *dst = a.y + static_cast<size_t>(tok) * a.out_f + row0 + r;
     *dst = a.accum ? *dst + sum : sum;
   }
 }
 
-template <int MT, int NT>
+template <int MT, int NT, int WARPS>
 wst_status_t launch_few(const FewArgs &a) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(static_cast<unsigned>((a.out_f + 16 * MT - 1) / (16 * MT)));
-  cfg.blockDim = dim3(kFewThreads);
+  cfg.blockDim = dim3(32 * WARPS);
   cfg.stream = current_stream();
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_int4_few_kernel<MT, NT>, a);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_int4_few_kernel<MT, NT, WARPS>, a);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail("wst_gemm_int4_hier (launch)", e);
   return WST_OK;
@@ -223,11 +220,17 @@ wst_status_t launch_gemm_int4_few(const void *qw, const void *si, const void *sb
   a.out_f = out_f;
   a.n = n;
   a.accum = accum;
-  /* 32 rows per CTA halve the x traffic; 16 when that would leave half the SMs without any */
+  /* Sixteen warps per SM that each walk little of K: with eight (32 rows per CTA, one CTA per SM)
+   * 5 tokens of 3584 -> 4608 took 9.7 us, with two CTAs of 16 rows 6.1; 4096 -> 6144 11.3 and
+   * 9.9.  From 9 tokens on 32 rows in one CTA of sixteen warps halve the x traffic where one
+   * wave takes them all: 16 tokens 12.2 -> 7.4 us, 8.1 with 16 rows; 4096 -> 6144 15.0 and 13.9
+   * before.  Few rows: sixteen warps on one CTA of 16 (896 -> 1152 2.4 -> 2.0). */
   const bool narrow = static_cast<long long>(out_f) < 16ll * sm_count;
-  if (n <= 8) return narrow ? launch_few<1, 1>(a) : launch_few<2, 1>(a);
-  if (n <= 16) return narrow ? launch_few<1, 2>(a) : launch_few<2, 2>(a);
-  return narrow ? launch_few<1, 4>(a) : launch_few<2, 4>(a);
+  const bool one_wave = static_cast<long long>(out_f) <= 32ll * sm_count;
+  if (n <= 8) return narrow ? launch_few<1, 1, 16>(a) : launch_few<1, 1, 8>(a);
+  if (n <= 16)
+    return narrow ? launch_few<1, 2, 16>(a) : one_wave ? launch_few<2, 2, 16>(a) : launch_few<2, 2, 8>(a);
+  return narrow ? launch_few<1, 4, 8>(a) : launch_few<2, 4, 8>(a);
 }
 
 }  // namespace wst
