@@ -141,7 +141,7 @@ __device__ __forceinline__ TokenPlace place_token(const RopeArgs &a, int tok) {
       p = p < 0 ? 0 : p;
       seq_base = static_cast<long long>(sq) * a.n_kv * a.max_seq * a.hd;
     } else if (a.pos_dev) {
-      p = *a.pos_dev;
+      p = __ldcg(a.pos_dev); /* not through L1: the hint below may have read an older value */
       p = p < 0 ? 0 : p;
     } else {
       p = a.pos0 + tok;
@@ -183,6 +183,18 @@ rope_append_kernel(const RopeArgs a) {
    * kernel in the stream (the decode attention, which re-reads the one row
    * written here after its own wait) start its prologue right away. */
   if (a.trigger_early && !PAGED) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  /* What bounds the single-token append is its chain of round trips to L2: cursor, table row at
+   * the cursor, values behind the rotated key.  The cursor is read once while the dependency is
+   * open, as a hint that may be out of date: behind the wait, the table row it names, the
+   * vectors and the cursor itself are asked for together, and the table row again if the cursor
+   * says otherwise. */
+  const bool guess = !PAGED && a.pos_dev != nullptr;
+  int hint = 0;
+  if (guess) {
+    hint = __ldcg(a.pos_dev);
+    const int top = min(a.max_seq, a.table_len) - 1;
+    hint = min(max(hint, 0), top);
+  }
   asm volatile("griddepcontrol.wait;" ::: "memory");
   /* paged (verify): the kernel behind reads the batch description and old cache rows
    * before its own dependency resolves, so it is released only now, when everything ahead
@@ -198,21 +210,35 @@ rope_append_kernel(const RopeArgs a) {
   const int tok = static_cast<int>(unit / heads);
   const int head = static_cast<int>(unit % heads);
 
-  const TokenPlace place = place_token<PAGED>(a, tok);
-  const int tpos = place.pos < a.table_len - 1 ? place.pos : a.table_len - 1;
-
   float *row = a.qkv + static_cast<long long>(tok) * (a.n_q + 2 * a.n_kv) * HD;
   const bool is_q = head < a.n_q;
   const int kvh = head - a.n_q;
   float *vec = is_q ? row + head * HD : row + (a.n_q + kvh) * HD;
+  const float *vsrc = row + (a.n_q + a.n_kv + kvh) * HD;
   const __half *gain = is_q ? a.q_gain : a.k_gain;
 
   const int i0 = lane * E;
-  float x1[E], x2[E], c[E], s[E];
+  float x1[E], x2[E], c[E], s[E], v1[E], v2[E], g1[E], g2[E];
   load_vec<E>(vec + i0, x1);
   load_vec<E>(vec + HALF + i0, x2);
-  load_vec<E>(a.cos_tab + static_cast<long long>(tpos) * HALF + i0, c);
-  load_vec<E>(a.sin_tab + static_cast<long long>(tpos) * HALF + i0, s);
+  if (guess) {
+    load_vec<E>(a.cos_tab + static_cast<long long>(hint) * HALF + i0, c);
+    load_vec<E>(a.sin_tab + static_cast<long long>(hint) * HALF + i0, s);
+  }
+  if (!is_q) {
+    load_vec<E>(vsrc + i0, v1);
+    load_vec<E>(vsrc + HALF + i0, v2);
+  }
+  if (gain) {
+    load_gain<E>(gain + i0, g1);
+    load_gain<E>(gain + HALF + i0, g2);
+  }
+  const TokenPlace place = place_token<PAGED>(a, tok);
+  const int tpos = place.pos < a.table_len - 1 ? place.pos : a.table_len - 1;
+  if (!guess || tpos != hint) {
+    load_vec<E>(a.cos_tab + static_cast<long long>(tpos) * HALF + i0, c);
+    load_vec<E>(a.sin_tab + static_cast<long long>(tpos) * HALF + i0, s);
+  }
 
   if (gain) {
     float ss = 0.f;
@@ -220,9 +246,6 @@ rope_append_kernel(const RopeArgs a) {
     for (int e = 0; e < E; ++e) ss = fmaf(x1[e], x1[e], fmaf(x2[e], x2[e], ss));
     ss = warp_sum(ss);
     const float inv = rsqrtf(ss / static_cast<float>(HD) + a.eps);
-    float g1[E], g2[E];
-    load_gain<E>(gain + i0, g1);
-    load_gain<E>(gain + HALF + i0, g2);
 #pragma unroll
     for (int e = 0; e < E; ++e) {
       x1[e] = x1[e] * inv * g1[e];
@@ -245,10 +268,6 @@ rope_append_kernel(const RopeArgs a) {
 
   if (place.kv_base < 0) return;
   const long long slot = place.kv_base + static_cast<long long>(kvh) * place.kv_head_stride;
-  const float *vsrc = row + (a.n_q + a.n_kv + kvh) * HD;
-  float v1[E], v2[E];
-  load_vec<E>(vsrc + i0, v1);
-  load_vec<E>(vsrc + HALF + i0, v2);
   if (a.kv8) { /* element offsets are byte offsets in an e4m3 cache */
     store_fp8_vec<E>(a.k_cache, slot + i0, y1, a.k_inv_scale);
     store_fp8_vec<E>(a.k_cache, slot + HALF + i0, y2, a.k_inv_scale);
