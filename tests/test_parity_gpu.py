@@ -543,6 +543,40 @@ def test_paged_prompts_beside_drafts(shape, lengths, counts):
         assert_close_per_head(got[cu_np[s]:cu_np[s + 1]], want, f"seq {s} ({L} + {c} rows)")
 
 
+def test_outputs_on_an_eight_byte_boundary():
+    """Buffers that the tensor-core tiles' 16-byte stores cannot take: drafts of one sequence and
+    a paged step with a prompt give what they give into aligned ones."""
+    shape, lengths, counts = workloads.QWEN25_7B, [300, 40], [3, 37]
+    n_q, n_kv, hd, theta = shape.n_q, shape.n_kv, shape.head_dim, 1e6
+    rng = np.random.default_rng(5)
+    width = n_q * hd
+
+    def both(numel, run):
+        plain = torch.zeros(numel, dtype=torch.float16, device="cuda")
+        odd = torch.zeros(numel + 4, dtype=torch.float16, device="cuda")[4:]
+        assert odd.data_ptr() % 16 == 8
+        run(plain)
+        run(odd)
+        assert_close_per_head(host(odd).astype(np.float64).reshape(-1, hd),
+                              host(plain).astype(np.float64).reshape(-1, hd), "8-byte boundary")
+
+    cache = decode.KvCache(n_kv, n_q, hd, 700)
+    cache.k[:, :600], cache.v[:, :600] = dev(rand16(rng, (n_kv, 600, hd))), dev(rand16(rng, (n_kv, 600, hd)))
+    qd = dev(workloads.f16_values(rng, (5, shape.qkv_width)))
+    both(5 * width, lambda out: chunk.attn(qd, cache, out, n_q, 595, 5))
+
+    pool, _, _, _ = build_paged_case(rng, shape, lengths, max(counts))
+    total, max_len = sum(counts), max(l + c for l, c in zip(lengths, counts))
+    rows = dev(workloads.f16_values(rng, (total, shape.qkv_width)))
+    pos0, cu = dev(np.asarray(lengths, np.int32)), dev(np.concatenate([[0], np.cumsum(counts)]).astype(np.int32))
+    paged.rope_cache(rows, pool, decode.RopeTable(max_len, hd, theta), n_q, pos0, cu, total)
+    scratch = torch.empty(paged.verify_scratch_floats(2, max(counts), n_q, n_kv, hd, max_len),
+                          dtype=torch.float32, device="cuda")
+    both(total * width, lambda out: paged.attn_verify(rows, pool, out, scratch, n_q, pos0, cu, total,
+                                                      max(counts), max_len))
+    assert decode.device_error() == 0
+
+
 # ------------------------------------------- bounded waits report, never hang
 
 def test_exchange_wait_runs_out_and_reports():

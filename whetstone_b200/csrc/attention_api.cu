@@ -527,11 +527,13 @@ extern "C" wst_status_t wst_attn_chunk(const void *qkv, const void *k_cache,
    * ahead even where most of their rows are empty: 2 tokens behind 4099 rows 10.8 us with the
    * append against 14.3 with the mma.sync row-block kernel, 5 tokens 12.1 and 19.3 (28 heads
    * over 4 of 128).  A single 16-row block streams better where the prefix is short (2 tokens
-   * behind 300 rows: 8.2 against 9.8) and at head_dim 64 (7.7 against 8.0). */
-  const bool one_block = n * (n_q / n_kv) <= 16;
-  const bool use_prefill = tc_ok && choice != 2 &&
-                     (choice == 3 || choice == 4 ? prefill_kernel_supports(n_q, n_kv, head_dim, n)
-                                                 : !one_block || (head_dim == 128 && pos0 + n > 512));
+   * behind 300 rows: 8.2 against 9.8) and at head_dim 64 (7.7 against 8.0); it also takes what
+   * the tiles' 16-byte stores cannot, `out` on a smaller boundary. */
+  const bool many = prefill_kernel_supports(n_q, n_kv, head_dim, n); /* at least 64 query rows */
+  const bool one_block = static_cast<long long>(n) * (n_q / n_kv) <= 16;
+  const bool few_in_tiles = choice == 0 && aligned16(out) &&
+                            (!one_block || (head_dim == 128 && pos0 + n > 512));
+  const bool use_prefill = tc_ok && choice != 2 && (many || few_in_tiles);
   int splits = 1;
   if (use_prefill && choice != 3 && choice != 4) {
     DeviceFacts facts;
@@ -740,8 +742,9 @@ extern "C" wst_status_t wst_attn_verify_paged(const void *qkv, const void *k_poo
   const bool one_tile = prefill_split_supports(n_q, n_kv, head_dim, max_tokens_per_seq);
   const long long verify_floats =
       wst_attn_verify_scratch_floats(n_seq, max_tokens_per_seq, n_q, n_kv, head_dim, max_len);
-  const bool span = choice != 3 && verify_span_fits(n_seq, max_tokens_per_seq, n_q, n_kv, head_dim,
-                                                    verify_floats);
+  /* (prompts with buffers on a smaller boundary stay with the row-block kernel, which takes them) */
+  const bool span = choice != 3 && (one_tile || (aligned16(out) && aligned16(scratch))) &&
+                    verify_span_fits(n_seq, max_tokens_per_seq, n_q, n_kv, head_dim, verify_floats);
   if (choice != 2 && (one_tile || span)) {
     DeviceFacts facts;
     if (!device_facts(&facts)) return WST_ERR_CUDA;
