@@ -53,7 +53,8 @@ struct PairCfg {
   static constexpr int OFF_EPI = OFF_PACK + NSLOT * SLOT_BYTES;
   static constexpr int OFF_BAR = OFF_EPI + 4 * EPI_WARP;
   static constexpr int NBAR = 2 * NSTAGE + 4 + 2 * NSLOT;
-  static constexpr int SMEM_BYTES = OFF_BAR + NBAR * 8 + 16 + 1024;
+  static constexpr int OFF_BOX = (OFF_BAR + NBAR * 8 + 4 + 15) / 16 * 16;
+  static constexpr int SMEM_BYTES = OFF_BOX + 16 + 1024;
   static constexpr int TMEM_COLS = 2 * BN;
   /* Unpacking warps on one stage, each with UNITS times eight rows, and sets of them that take
    * the stages in turn: with all sixteen on one stage (BN = 256, one unit each) they waited,
@@ -79,12 +80,41 @@ __device__ __forceinline__ uint32_t in_leader(uint32_t addr) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(addr));
   return r;
 }
-/* Arrives on a barrier of either CTA of the pair.  What it announces -- shared memory written
- * and fenced towards the async proxy, tensor memory read -- lies in this SM, and the MMA that
- * waits for it reads or writes it in this SM; a release at cluster scope made every arrival
- * wait for the thread's memory traffic, 0.9 us of a stage. */
-__device__ __forceinline__ void mbar_arrive_pair(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+/* Tells the pair's first CTA, by 16 bytes that its barrier counts, that what this thread has seen
+ * happen in its own CTA has happened: the copy is issued behind that, and its completion is a
+ * release at cluster scope.  (An arrival with such a release is as sound but makes the arriving
+ * thread wait for the SM's memory traffic, 0.5 to 0.9 us each: 256 tokens of 3584 -> 4608, int4
+ * weights, 14.9 us with messages and 28 with one arrival a stage.) */
+constexpr int kMessage = 16;
+__device__ __forceinline__ void tell_leader(uint32_t mailbox, uint32_t src, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+      ::"r"(in_leader(mailbox)), "r"(src), "n"(kMessage), "r"(in_leader(bar))
+      : "memory");
+}
+__device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity) {
+  uint32_t done;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(done)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return done != 0;
+}
+/* mbar_wait for what the other CTA announces */
+__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, unsigned int *err_word,
+                                                  unsigned int code) {
+  if (mbar_try_wait_cluster(bar, parity)) return true;
+  const long long t0 = clock64();
+  while (!mbar_try_wait_cluster(bar, parity)) {
+    if (clock64() - t0 > kWaitCycleLimit) {
+      if (err_word) atomicCAS(err_word, 0u, code);
+      return false;
+    }
+  }
+  return true;
 }
 __device__ __forceinline__ void pair_tmem_alloc(uint32_t dst_smem, uint32_t cols) {
   asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_smem),
@@ -245,22 +275,26 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
   const uint32_t sbase = smem_u32(smem);
   const uint32_t bar0 = sbase + C::OFF_BAR;
   auto bar = [bar0](int i) { return bar0 + 8u * i; };
-  /* FULL and ACC_EMPTY count in the leader, EMPTY and ACC_FULL in each CTA */
+  /* EMPTY and ACC_FULL: the leader's MMAs announce them in each CTA.  FULL and ACC_EMPTY: what a
+   * CTA's own threads have done for its half of a tile is counted in that CTA; the second CTA's
+   * idle MMA warp waits there and tells the leader's barrier. */
   constexpr int FULL = 0, EMPTY = NSTAGE, ACC_FULL = 2 * NSTAGE, ACC_EMPTY = ACC_FULL + 2;
   constexpr int P_FULL = ACC_EMPTY + 2, P_EMPTY = P_FULL + C::NSLOT;
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + C::OFF_BAR + C::NBAR * 8);
+  const uint32_t mailbox = sbase + C::OFF_BOX; /* of messages: nobody reads it */
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = static_cast<int>(cluster_rank());
   const PairGemm &g = a.g;
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < NSTAGE; ++i) {
-      mbar_init(bar(FULL + i), INT4 ? 1 + 2 * C::STAGE_WARPS : 1);
+      /* leader: the announcement of the bytes; either: its own unpacking warps */
+      mbar_init(bar(FULL + i), !INT4 ? 1 : rank == 0 ? 1 + C::STAGE_WARPS : C::STAGE_WARPS);
       mbar_init(bar(EMPTY + i), 1);
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(bar(ACC_FULL + i), 1);
-      mbar_init(bar(ACC_EMPTY + i), 8);
+      mbar_init(bar(ACC_EMPTY + i), 4);
     }
     for (int i = 0; i < C::NSLOT; ++i) {
       mbar_init(bar(P_FULL + i), 1 + 32); /* the words' request, each lane's scale bytes */
@@ -301,9 +335,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
             ok = false;
             break;
           }
-          /* the leader's barrier counts the bytes of both CTAs */
+          /* the leader's barrier counts the bytes of both CTAs, and the message that the second
+           * CTA's weights are unpacked */
           if (rank == 0)
-            mbar_arrive_expect_tx(bar(FULL + st), 2 * (INT4 ? C::A_BYTES : C::STAGE_BYTES));
+            mbar_arrive_expect_tx(bar(FULL + st), INT4 ? 2 * C::A_BYTES + kMessage : 2 * C::STAGE_BYTES);
           const uint32_t full = in_leader(bar(FULL + st));
           const uint32_t dst = sbase + st * C::STAGE_BYTES;
 #pragma unroll
@@ -368,7 +403,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
         fence_async_smem();
         __syncwarp();
         if (lane == 0) {
-          mbar_arrive_pair(in_leader(bar(FULL + st)));
+          mbar_arrive(bar(FULL + st));
           mbar_arrive(bar(P_EMPTY + sl));
         }
         kb += C::SETS;
@@ -379,7 +414,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
       }
     }
   } else if (warp == 4) {
-    /* ------------------------------------------------ MMA issuer, the leader's only */
+    /* ------------------------------------------------ MMA issuer, in the leader */
     if (rank == 0) {
       constexpr uint32_t idesc = umma_idesc(256, BN, 0);
       int it = 0, local = 0;
@@ -388,11 +423,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
         const int buf = local & 1;
         /* both CTAs' epilogues of the tile two back have emptied this accumulator */
         if (local >= 2 &&
-            !mbar_wait(bar(ACC_EMPTY + buf), ((local >> 1) - 1) & 1, a.err_word, 0x702u)) break;
+            !mbar_wait_cluster(bar(ACC_EMPTY + buf), ((local >> 1) - 1) & 1, a.err_word, 0x702u)) break;
         tc_fence_after_sync();
         for (int kb = 0; kb < k_blocks; ++kb, ++it) {
           const int st = it % NSTAGE;
-          if (!mbar_wait(bar(FULL + st), (it / NSTAGE) & 1, a.err_word, 0x703u)) { ok = false; break; }
+          if (!mbar_wait_cluster(bar(FULL + st), (it / NSTAGE) & 1, a.err_word, 0x703u)) { ok = false; break; }
           tc_fence_after_sync();
           const uint32_t a_lo = umma_desc_lo(sbase + st * C::STAGE_BYTES, 16);
           const uint32_t b_lo = umma_desc_lo(sbase + st * C::STAGE_BYTES + C::A_BYTES, 16);
@@ -408,6 +443,27 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
             if (kb == k_blocks - 1) pair_umma_commit(bar(ACC_FULL + buf));
           }
           __syncwarp();
+        }
+      }
+    } else if (lane == 0) {
+      /* ------------ the second CTA: passes its accumulators and weight tiles on, in the order in
+       * which the leader waits for them */
+      int it = 0, local = 0;
+      bool ok = true;
+      for (int tile = first_tile; ok && tile < n_tiles_total; tile += tile_step, ++local) {
+        const int buf = local & 1;
+        if (local >= 2) {
+          if (!mbar_wait(bar(ACC_EMPTY + buf), ((local >> 1) - 1) & 1, a.err_word, 0x70Au)) break;
+          tc_fence_after_sync();
+          tc_fence_before_sync();
+          tell_leader(mailbox, mailbox, bar(ACC_EMPTY + buf));
+        }
+        if constexpr (INT4) {
+          for (int kb = 0; kb < k_blocks; ++kb, ++it) {
+            const int st = it % NSTAGE;
+            if (!mbar_wait(bar(FULL + st), (it / NSTAGE) & 1, a.err_word, 0x70Bu)) { ok = false; break; }
+            tell_leader(mailbox, sbase + st * C::STAGE_BYTES + C::A_BYTES, bar(FULL + st));
+          }
         }
       }
     }
@@ -511,7 +567,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
       }
       tc_fence_before_sync();
       __syncwarp();
-      if (lane == 0) mbar_arrive_pair(in_leader(bar(ACC_EMPTY + buf)));
+      if (lane == 0) {
+        if (rank == 0 && warp == 0) mbar_arrive_expect_tx(bar(ACC_EMPTY + buf), kMessage);
+        else mbar_arrive(bar(ACC_EMPTY + buf));
+      }
     }
     grid_launch_dependents();
   }
