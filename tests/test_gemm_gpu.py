@@ -217,3 +217,20 @@ def test_up_to_128_tokens_at_the_edges_of_the_row_choices(in_f, out_f, n):
     x = rng.standard_normal((n, in_f)).astype(np.float16)
     y0 = rng.standard_normal((n, out_f)).astype(np.float32)
     close(run(w, x, None, y0, True), orc.gemm_fp16(w, x, None, y0), 2e-4, f"{in_f} x {out_f} x {n}")
+
+
+@pytest.mark.parametrize("in_f", [64, 128, 200, 392, 520])   # fewer, as many and more stages than the ring
+def test_projections_that_follow_each_other_at_once(in_f):
+    """Launch after launch on the same SMs, K from one stage up: nothing that a launch's last
+    MMAs still signal reaches the barriers of the next."""
+    rng = np.random.default_rng(in_f)
+    out_f, n = 768, 520
+    w, x = dev((rng.standard_normal((out_f, in_f)) / np.sqrt(in_f)).astype(np.float16)), \
+        dev(rng.standard_normal((n, in_f)).astype(np.float16))
+    ys = [torch.full((n, out_f), float("nan"), dtype=torch.float32, device="cuda") for _ in range(40)]
+    for y in ys:
+        chunk.gemm_fp16(w, x, None, y, in_f, out_f, n)
+    torch.cuda.synchronize()
+    assert decode.device_error() == 0
+    close(host(ys[0]), orc.gemm_fp16(host(w), host(x)), 2e-4, f"in_f {in_f}")
+    assert all(torch.equal(y, ys[0]) for y in ys)

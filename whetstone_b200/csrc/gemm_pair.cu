@@ -349,6 +349,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
           }
         }
       }
+      /* the last uses' commits arrive here, from the leader's MMAs: not after this CTA is gone */
+      for (int u = it > NSTAGE ? it - NSTAGE : 0; ok && u < it; ++u)
+        ok = mbar_wait(bar(EMPTY + u % NSTAGE), (u / NSTAGE) & 1, a.err_word, 0x709u);
     }
   } else if (INT4 && warp == 6) {
     /* -------------------------------- packed words and scale bytes of this CTA's rows */
