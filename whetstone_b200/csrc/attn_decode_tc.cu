@@ -384,7 +384,7 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
         uint32_t qp[32];
 #pragma unroll
         for (int e = 0; e < 32; e += 2) {
-          const float4 f = __ldg(reinterpret_cast<const float4 *>(src + 2 * (c0 + e)));
+          const float4 f = *reinterpret_cast<const float4 *>(src + 2 * (c0 + e));
           qp[e] = valid ? pack_half2(f.x * a.qscale, f.y * a.qscale) : 0u;
           qp[e + 1] = valid ? pack_half2(f.z * a.qscale, f.w * a.qscale) : 0u;
         }

@@ -380,7 +380,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap kmap,
       if (valid && a.q16) {
 #pragma unroll
         for (int e = 0; e < QC; e += 2) {
-          const uint2 h = __ldg(reinterpret_cast<const uint2 *>(src16 + 2 * e));
+          const uint2 h = *reinterpret_cast<const uint2 *>(src16 + 2 * e);
           const float2 lo = __half22float2(*reinterpret_cast<const __half2 *>(&h.x));
           const float2 hi = __half22float2(*reinterpret_cast<const __half2 *>(&h.y));
           packed[e] = pack_half2(lo.x * a.qscale, lo.y * a.qscale);
@@ -390,7 +390,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap kmap,
 #pragma unroll
         for (int e = 0; e < QC; e += 2) {
           float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (valid) f = __ldg(reinterpret_cast<const float4 *>(src + 2 * e));
+          if (valid) f = *reinterpret_cast<const float4 *>(src + 2 * e);
           packed[e] = pack_half2(f.x * a.qscale, f.y * a.qscale);
           packed[e + 1] = pack_half2(f.z * a.qscale, f.w * a.qscale);
         }
@@ -866,33 +866,39 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap kmap,
       /* one loop per source type: with the choice inside the loop the loads of the eight
        * rows no longer went out together and a launch took 13 us longer */
       auto stage_rows = [&](auto load_row) {
-#pragma unroll 8
-        for (int i = 0; i < 32 / RPI; ++i) {
-          float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (row < rows_valid) v = load_row(tok * a.q_tok_stride + head * HD);
-          uint2 h;
-          h.x = pack_half2(v.x * a.qscale, v.y * a.qscale);
-          h.y = pack_half2(v.z * a.qscale, v.w * a.qscale);
-          *reinterpret_cast<uint2 *>(q_smem + swz128(row, (l >> 1) & 7)) = h;
-          row += RPI;
-          head += RPI;
-          if (head >= a.gqa) { /* RPI <= 2: one step at most when gqa >= RPI */
-            head -= a.gqa;
-            ++tok;
-            if (head >= a.gqa) { head -= a.gqa; ++tok; }
+#pragma unroll 1
+        for (int i = 0; i < 32 / RPI; i += 8) {
+          float4 v[8]; /* all eight asked for before any is stored */
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (row + k * RPI < rows_valid) v[k] = load_row(tok * a.q_tok_stride + head * HD);
+            head += RPI;
+            if (head >= a.gqa) { /* RPI <= 2: one step at most when gqa >= RPI */
+              head -= a.gqa;
+              ++tok;
+              if (head >= a.gqa) { head -= a.gqa; ++tok; }
+            }
+          }
+#pragma unroll
+          for (int k = 0; k < 8; ++k, row += RPI) {
+            uint2 h;
+            h.x = pack_half2(v[k].x * a.qscale, v[k].y * a.qscale);
+            h.y = pack_half2(v[k].z * a.qscale, v[k].w * a.qscale);
+            *reinterpret_cast<uint2 *>(q_smem + swz128(row, (l >> 1) & 7)) = h;
           }
         }
       };
       if (a.q16) {
         stage_rows([&](long long off) {
-          const uint2 h = __ldg(reinterpret_cast<const uint2 *>(q16_tile + off));
+          const uint2 h = *reinterpret_cast<const uint2 *>(q16_tile + off);
           const float2 lo = __half22float2(*reinterpret_cast<const __half2 *>(&h.x));
           const float2 hi = __half22float2(*reinterpret_cast<const __half2 *>(&h.y));
           return make_float4(lo.x, lo.y, hi.x, hi.y);
         });
       } else {
         stage_rows([&](long long off) {
-          return __ldg(reinterpret_cast<const float4 *>(q_tile + off));
+          return *reinterpret_cast<const float4 *>(q_tile + off);
         });
       }
       fence_async_smem();
@@ -1506,7 +1512,7 @@ attn_verify_span_kernel(const __grid_constant__ CUtensorMap kmap,
 #pragma unroll
       for (int e = 0; e < QC; e += 2) {
         float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (valid) f = __ldg(reinterpret_cast<const float4 *>(src + 2 * e));
+        if (valid) f = *reinterpret_cast<const float4 *>(src + 2 * e);
         packed[e] = pack_half2(f.x * a.qscale, f.y * a.qscale);
         packed[e + 1] = pack_half2(f.z * a.qscale, f.w * a.qscale);
       }

@@ -292,8 +292,8 @@ attn_rows_kernel(const __grid_constant__ CUtensorMap kmap,
         const float4 *src = reinterpret_cast<const float4 *>(
             a.q + static_cast<long long>(tok) * a.q_tok_stride +
             static_cast<long long>(head) * HD + ch * 8);
-        lo[it] = __ldg(src);
-        hi[it] = __ldg(src + 1);
+        lo[it] = src[0];
+        hi[it] = src[1];
       }
     }
 #pragma unroll

@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(32 * WARPS, 16 / WARPS) gemm_int4_few_kernel(c
     const int grp = 4 * s + t;
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt)
-      d[nt] = grp < groups ? __ldg(reinterpret_cast<const uint4 *>(xrow[nt] + grp * 32) + wi)
+      d[nt] = grp < groups ? reinterpret_cast<const uint4 *>(xrow[nt] + grp * 32)[wi]
                            : make_uint4(0u, 0u, 0u, 0u);
   };
   /* word `wi` of the rows' groups: unpacked, multiplied */
