@@ -219,6 +219,32 @@ def test_up_to_128_tokens_at_the_edges_of_the_row_choices(in_f, out_f, n):
     close(run(w, x, None, y0, True), orc.gemm_fp16(w, x, None, y0), 2e-4, f"{in_f} x {out_f} x {n}")
 
 
+@pytest.mark.parametrize("n", [5, 24, 80, 200])   # each kernel of either weight format
+@pytest.mark.parametrize("weights", ["fp16", "int4"])
+def test_accumulating_keeps_numbers_below_the_normal_range(weights, n):
+    """y + v as fp32 adds them, bit for bit, where y lies below 2^-126: v is zero, or cancels
+    y or outweighs it (fp16 weights: every third feature)."""
+    in_f, out_f = 256, 320
+    y0 = (np.random.default_rng(n).uniform(-1.0, 1.0, (n, out_f)) * 1e-38).astype(np.float32)
+    assert (np.abs(y0) < np.finfo(np.float32).tiny).any()
+    x, want = dev(np.ones((n, in_f), np.float16)), y0.copy()
+    w = np.zeros((out_f, in_f), np.float16)
+    if weights == "fp16":
+        w[::3, 0] = 2.0 ** -14
+        y0[:, ::6] = -(2.0 ** -14)
+        want[:, ::3] = y0[:, ::3] + np.float32(2.0 ** -14)
+    y = dev(y0)
+    if weights == "fp16":
+        chunk.gemm_fp16(dev(w), x, None, y, in_f, out_f, n, True)
+    else:
+        groups = out_f * in_f // 32
+        chunk.gemm_int4_hier(dev(np.zeros(groups * 4, np.int32)), dev(np.zeros(groups, np.uint8)),
+                             dev(np.zeros((out_f, 2), np.float16)), x, None, y, in_f, out_f, n, True)
+    torch.cuda.synchronize()
+    assert decode.device_error() == 0
+    assert (host(y).view(np.uint32) == want.view(np.uint32)).all()
+
+
 @pytest.mark.parametrize("in_f", [64, 128, 200, 392, 520])   # fewer, as many and more stages than the ring
 def test_projections_that_follow_each_other_at_once(in_f):
     """Launch after launch on the same SMs, K from one stage up: nothing that a launch's last
