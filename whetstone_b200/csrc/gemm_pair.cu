@@ -343,7 +343,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
         for (int kb = 0; kb < k_blocks; ++kb, ++it) {
           const int st = it % NSTAGE;
           if (it >= NSTAGE &&
-              !mbar_wait(bar(EMPTY + st), ((it / NSTAGE) - 1) & 1, a.err_word, 0x701u)) {
+              !mbar_wait(bar(EMPTY + st), ((it / NSTAGE) - 1) & 1, a.err_word, 0x901u)) {
             ok = false;
             break;
           }
@@ -363,7 +363,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
       }
       /* the last uses' commits arrive here, from the leader's MMAs: not after this CTA is gone */
       for (int u = it > NSTAGE ? it - NSTAGE : 0; ok && u < it; ++u)
-        ok = mbar_wait(bar(EMPTY + u % NSTAGE), (u / NSTAGE) & 1, a.err_word, 0x709u);
+        ok = mbar_wait(bar(EMPTY + u % NSTAGE), (u / NSTAGE) & 1, a.err_word, 0x909u);
     }
   } else if (INT4 && warp == 6) {
     /* -------------------------------- packed words and scale bytes of this CTA's rows */
@@ -376,7 +376,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
         for (int kb = 0; kb < k_blocks; ++kb, ++it) {
           const int sl = it % C::NSLOT;
           if (it >= C::NSLOT) {
-            const bool free = mbar_wait(bar(P_EMPTY + sl), ((it / C::NSLOT) - 1) & 1, a.err_word, 0x707u);
+            const bool free = mbar_wait(bar(P_EMPTY + sl), ((it / C::NSLOT) - 1) & 1, a.err_word, 0x907u);
             if (!__all_sync(0xffffffffu, free)) { ok = false; break; }
           }
           packed.fetch(sbase + C::OFF_PACK + sl * C::SLOT_BYTES, bar(P_FULL + sl), kb, lane);
@@ -408,8 +408,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
       bool ok = true;
       for (int it = set; ok && it < total; it += C::SETS) {
         const int st = it % NSTAGE, sl = it % C::NSLOT;
-        ok = mbar_wait(bar(P_FULL + sl), (it / C::NSLOT) & 1, a.err_word, 0x708u) &&
-             (it < NSTAGE || mbar_wait(bar(EMPTY + st), ((it / NSTAGE) - 1) & 1, a.err_word, 0x705u));
+        ok = mbar_wait(bar(P_FULL + sl), (it / C::NSLOT) & 1, a.err_word, 0x908u) &&
+             (it < NSTAGE || mbar_wait(bar(EMPTY + st), ((it / NSTAGE) - 1) & 1, a.err_word, 0x905u));
         if (!__all_sync(0xffffffffu, ok)) break;
         const uint8_t *slot = smem + C::OFF_PACK + sl * C::SLOT_BYTES;
 #pragma unroll
@@ -438,11 +438,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
         const int buf = local & 1;
         /* both CTAs' epilogues of the tile two back have emptied this accumulator */
         if (local >= 2 &&
-            !mbar_wait_cluster(bar(ACC_EMPTY + buf), ((local >> 1) - 1) & 1, a.err_word, 0x702u)) break;
+            !mbar_wait_cluster(bar(ACC_EMPTY + buf), ((local >> 1) - 1) & 1, a.err_word, 0x902u)) break;
         tc_fence_after_sync();
         for (int kb = 0; kb < k_blocks; ++kb, ++it) {
           const int st = it % NSTAGE;
-          if (!mbar_wait_cluster(bar(FULL + st), (it / NSTAGE) & 1, a.err_word, 0x703u)) { ok = false; break; }
+          if (!mbar_wait_cluster(bar(FULL + st), (it / NSTAGE) & 1, a.err_word, 0x903u)) { ok = false; break; }
           tc_fence_after_sync();
           const uint32_t a_lo = umma_desc_lo(sbase + st * C::STAGE_BYTES, 16);
           const uint32_t b_lo = umma_desc_lo(sbase + st * C::STAGE_BYTES + C::A_BYTES, 16);
@@ -468,7 +468,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
       for (int tile = first_tile; ok && tile < n_tiles_total; tile += tile_step, ++local) {
         const int buf = local & 1;
         if (local >= 2) {
-          if (!mbar_wait(bar(ACC_EMPTY + buf), ((local >> 1) - 1) & 1, a.err_word, 0x70Au)) break;
+          if (!mbar_wait(bar(ACC_EMPTY + buf), ((local >> 1) - 1) & 1, a.err_word, 0x90Au)) break;
           tc_fence_after_sync();
           tc_fence_before_sync();
           tell_leader(mailbox, mailbox, bar(ACC_EMPTY + buf));
@@ -476,7 +476,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
         if constexpr (INT4) {
           for (int kb = 0; kb < k_blocks; ++kb, ++it) {
             const int st = it % NSTAGE;
-            if (!mbar_wait(bar(FULL + st), (it / NSTAGE) & 1, a.err_word, 0x70Bu)) { ok = false; break; }
+            if (!mbar_wait(bar(FULL + st), (it / NSTAGE) & 1, a.err_word, 0x90Bu)) { ok = false; break; }
             tell_leader(mailbox, sbase + st * C::STAGE_BYTES + C::A_BYTES, bar(FULL + st));
           }
         }
@@ -491,7 +491,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
     for (int tile = first_tile; tile < n_tiles_total; tile += tile_step, ++local) {
       const int buf = local & 1;
       const int m0 = (tile % a.m_tiles) * 256 + rank * 128, n0 = (tile / a.m_tiles) * BN;
-      if (!mbar_wait_idle(bar(ACC_FULL + buf), (local >> 1) & 1, a.err_word, 0x704u)) break;
+      if (!mbar_wait_idle(bar(ACC_FULL + buf), (local >> 1) & 1, a.err_word, 0x904u)) break;
       tc_fence_after_sync();
       const uint32_t acc = tmem + lane_base + buf * BN;
       if constexpr (ROPE) {
