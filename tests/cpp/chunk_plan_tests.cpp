@@ -1,0 +1,58 @@
+/* CPU-only checks of the arithmetic that cuts a chunk's KV range and picks its kernel
+ * (whetstone_b200/csrc/chunk_plan.hpp). */
+#include <cstdio>
+#include <initializer_list>
+
+#include "chunk_plan.hpp"
+
+using namespace wst;
+
+static int failures = 0;
+#define CHECK(cond, ...)                                          \
+  do {                                                            \
+    if (!(cond)) {                                                \
+      std::printf("FAILED %s:%d: %s  ", __FILE__, __LINE__, #cond); \
+      std::printf(__VA_ARGS__);                                   \
+      std::printf("\n");                                          \
+      ++failures;                                                 \
+    }                                                             \
+  } while (0)
+
+constexpr int kSms = 148;
+static int up(int a, int b) { return (a + b - 1) / b; }
+
+/* heads of a group, KV heads, tokens, positions: every tile in one slice, no slice without one,
+ * no launch of more CTAs than SMs */
+static void slices_cover_the_prefix_and_none_is_empty() {
+  for (int gqa : {1, 4, 7, 8, 64})
+    for (int n_kv : {1, 2, 4, 8, 32})
+      for (int n : {1, 2, 5, 9, 18, 19, 64, 73, 128, 256, 512})
+        for (int len = n; len <= 40000; len = len < 1100 ? len + 1 : len + 61) {
+          const long long tiles = static_cast<long long>(up(n * gqa, 128)) * n_kv;
+          const int s = chunk_slices(kSms, tiles, len, true);
+          if (s == 1) continue;
+          const int kv = up(len, kKvTile), each = slice_tiles(len, s);
+          CHECK(s <= kMaxChunkSlices && s * tiles <= kSms, "%d slices of %lld tiles", s, tiles);
+          CHECK(s * each >= kv && (s - 1) * each < kv, "%d slices of %d for %d tiles, len %d", s, each, kv, len);
+        }
+}
+
+/* either side of a KV tile's end the same prefix is cut the same way */
+static void a_prefix_that_ends_with_a_tile_is_cut_like_its_neighbours() {
+  for (int tiles : {1, 2, 4, 8})
+    for (int len = 512; len <= 4096; len += 128) {
+      const int s = chunk_slices(kSms, tiles, len, true);
+      CHECK(s == chunk_slices(kSms, tiles, len - 1, true), "len %d", len);
+      CHECK(slice_tiles(len, s) == slice_tiles(len - 1, s), "len %d", len);
+    }
+  /* 28 heads over 4, 5 tokens, 4096 positions: 32 KV tiles in 32 slices */
+  const int s = chunk_slices(kSms, 4, 4096, true);
+  CHECK(s == 32 && slice_tiles(4096, s) == 1, "%d slices of %d", s, slice_tiles(4096, s));
+}
+
+int main() {
+  slices_cover_the_prefix_and_none_is_empty();
+  a_prefix_that_ends_with_a_tile_is_cut_like_its_neighbours();
+  std::printf(failures ? "%d failures\n" : "chunk plan ok\n", failures);
+  return failures != 0;
+}

@@ -23,6 +23,13 @@ def test_cpp_paged_kv_manager_tests_pass():
     assert proc.returncode == 0 and "0 failed" in proc.stdout, proc.stdout + proc.stderr
 
 
+def test_cpp_chunk_plan_tests_pass():
+    """tests/cpp/chunk_plan_tests.cpp: how a chunk's KV range is cut (no GPU)."""
+    subprocess.run(["make", "-C", str(ROOT / "tests" / "cpp")], check=True, capture_output=True)
+    proc = subprocess.run([str(BIN.parent / "chunk_plan_tests")], capture_output=True, text=True, timeout=60)
+    assert proc.returncode == 0 and "chunk plan ok" in proc.stdout, proc.stdout + proc.stderr
+
+
 @pytest.mark.gpu
 def test_cpp_kernel_tests_pass():
     if not BIN.exists():

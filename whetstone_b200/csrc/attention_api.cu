@@ -7,10 +7,13 @@
 
 #include "attn_prefill.cuh"
 #include "attn_rows.cuh"
+#include "chunk_plan.hpp"
 #include "wst_ptx.cuh"
 
 namespace wst {
 namespace {
+
+static_assert(kMaxChunkSlices == kRowsMaxSplits, "what the merge takes");
 
 std::atomic<int> g_kernel_choice{0};
 
@@ -59,23 +62,6 @@ float *chunk_workspace(const char **why) {
 void note_unsplit(const char *who, const char *why) {
   fail(WST_OK, "%s: ran without splitting the KV range (%s); call "
                "wst_b200_reserve_chunk_workspace once outside any capture", who, why);
-}
-
-/* Slices of the KV range for a chunk launch of `tiles` (unit, query tile) pairs against at
- * most `len` positions: none when the tiles fill the GPU by themselves or the prefix is short;
- * else enough to fill it, in runs of at least two KV tiles.  A few rows cost the merge little:
- * for them down to one KV tile each, behind 256 rows already (append and attention, 28 heads
- * over 4 of 128: 5 tokens behind 4099 rows 12.1 us with 33 slices, 13.9 with 16; behind 450
- * rows 9.8 and 11.6 unsplit.  128 tokens behind 1000 rows: 22.4 in runs of two, 23.3 of one;
- * 256 tokens behind none or 256: 17.1 unsplit, 19.6 split). */
-int chunk_slices(int sm_count, long long tiles, int len) {
-  const bool few = tiles <= 8;
-  if (tiles <= 0 || tiles * 2 > sm_count || len <= (few ? 256 : 512)) return 1;
-  long long s = sm_count / tiles;
-  const long long most = (len + 127) / 128 / (few ? 1 : 2);
-  if (s > most) s = most;
-  if (s > kRowsMaxSplits) s = kRowsMaxSplits;
-  return s < 2 ? 1 : static_cast<int>(s);
 }
 
 int max_splits_for(int max_seq) {
@@ -539,7 +525,7 @@ extern "C" wst_status_t wst_attn_chunk(const void *qkv, const void *k_cache,
     DeviceFacts facts;
     if (!device_facts(&facts)) return WST_ERR_CUDA;
     splits = chunk_slices(facts.sm_count,
-                          (static_cast<long long>(n) * (n_q / n_kv) + 127) / 128 * n_kv, pos0 + n);
+                          (static_cast<long long>(n) * (n_q / n_kv) + 127) / 128 * n_kv, pos0 + n, true);
   }
   if (use_prefill) {
     PrefillLaunch P;
@@ -636,7 +622,7 @@ static wst_status_t chunk_batch_common(const void *qkv, bool q16, const void *k_
       if (!device_facts(&facts)) return WST_ERR_CUDA;
       const int gqa = n_q / n_kv;
       const int splits = chunk_slices(
-          facts.sm_count, (static_cast<long long>(n) * gqa + 127) / 128 * n_kv * n_seq, max_seq);
+          facts.sm_count, (static_cast<long long>(n) * gqa + 127) / 128 * n_kv * n_seq, max_seq, false);
       if (splits > 1) {
         const char *why = "";
         P.scratch = chunk_workspace(&why);

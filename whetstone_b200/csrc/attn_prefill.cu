@@ -35,6 +35,7 @@
 
 #include "attn_prefill.cuh"
 #include "attn_rows.cuh"
+#include "chunk_plan.hpp"
 #include "tensor_map.cuh"
 #include "wst_ptx.cuh"
 
@@ -1912,8 +1913,7 @@ wst_status_t launch_prefill(const PrefillLaunch &P) {
          units * a.n_qtiles * splits * a.rows_cap * (P.hd + 4) > P.scratch_floats)
     --splits;
   a.n_splits = splits;
-  const int max_tiles = (P.max_len > 0 ? P.max_len : P.max_seq) / 128 + 1;
-  a.tiles_per_slice = splits > 1 && !P.even_slices ? (max_tiles + splits - 1) / splits : 0;
+  a.tiles_per_slice = splits > 1 && !P.even_slices ? slice_tiles(P.max_len > 0 ? P.max_len : P.max_seq, splits) : 0;
 
   CUtensorMap kmap, vmap;
   KvMapKey key{};
