@@ -28,7 +28,7 @@ static void slices_cover_the_prefix_and_none_is_empty() {
     for (int n_kv : {1, 2, 4, 8, 32})
       for (int n : {1, 2, 5, 9, 18, 19, 64, 73, 128, 256, 512})
         for (int len = n; len <= 40000; len = len < 1100 ? len + 1 : len + 61) {
-          const long long tiles = static_cast<long long>(up(n * gqa, 128)) * n_kv;
+          const long long tiles = query_tiles(n, gqa) * n_kv;
           const int s = chunk_slices(kSms, tiles, len, true);
           if (s == 1) continue;
           const int kv = up(len, kKvTile), each = slice_tiles(len, s);
@@ -46,13 +46,22 @@ static void a_prefix_that_ends_with_a_tile_is_cut_like_its_neighbours() {
       CHECK(slice_tiles(len, s) == slice_tiles(len - 1, s), "len %d", len);
     }
   /* 28 heads over 4, 5 tokens, 4096 positions: 32 KV tiles in 32 slices */
-  const int s = chunk_slices(kSms, 4, 4096, true);
+  const int s = chunk_slices(kSms, query_tiles(5, 7) * 4, 4096, true);
   CHECK(s == 32 && slice_tiles(4096, s) == 1, "%d slices of %d", s, slice_tiles(4096, s));
+}
+
+/* tiles hold whole tokens: 18 of seven heads, not 128 rows */
+static void query_tiles_are_the_kernels_own() {
+  CHECK(query_tiles(73, 7) == 5, "%lld", query_tiles(73, 7));
+  CHECK(query_tiles(18, 7) == 1 && query_tiles(19, 7) == 2, "18 tokens fill one");
+  CHECK(query_tiles(32, 4) == 1 && query_tiles(33, 4) == 2, "32 tokens fill one");
+  CHECK(query_tiles(3, 64) == 2, "two tokens fill one");
 }
 
 int main() {
   slices_cover_the_prefix_and_none_is_empty();
   a_prefix_that_ends_with_a_tile_is_cut_like_its_neighbours();
+  query_tiles_are_the_kernels_own();
   std::printf(failures ? "%d failures\n" : "chunk plan ok\n", failures);
   return failures != 0;
 }

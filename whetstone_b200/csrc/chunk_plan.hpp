@@ -7,22 +7,33 @@ namespace wst {
 constexpr int kKvTile = 128;       /* positions per KV tile of the tcgen05 kernels */
 constexpr int kMaxChunkSlices = 64;
 
+/* A query tile is up to 128 rows, whole tokens with all the heads of a KV head's group. */
+inline long long query_tiles(int n, int gqa) {
+  const int tokens = 128 / gqa;
+  return (static_cast<long long>(n) + tokens - 1) / tokens;
+}
+
 /* KV tiles of a slice when `len` positions are cut into `slices` runs; the last may be shorter. */
 inline int slice_tiles(int len, int slices) {
   const int tiles = (len + kKvTile - 1) / kKvTile;
   return (tiles + slices - 1) / slices;
 }
 
-/* Slices of the KV range for a chunk launch of `tiles` (unit, query tile) pairs against at
- * most `len` positions: none when the tiles fill the GPU by themselves or the prefix is short;
- * else enough to fill it, in runs of at least two KV tiles.  A few rows cost the merge little:
- * for them down to one KV tile each, behind 256 rows already (append and attention, 28 heads
- * over 4 of 128, caches from HBM: 5 tokens behind 500 rows 10.6 us in four slices, 11.7 in two, 12.5
- * unsplit.  128 tokens behind 1000 rows: 22.4 in runs of two, 23.3 of one; 256 tokens behind none
- * or 256: 17.1 unsplit, 19.6 split).  `exact`: `len` is the prefix, not the capacity of a cache. */
+/* Slices of the KV range for a chunk launch of `tiles` (unit, query tile) pairs against `len`
+ * positions: none when the tiles fill the GPU by themselves or the prefix is short; else enough to
+ * fill it, in runs of at least two KV tiles.  Up to sixteen tiles, full or not, leave so many SMs
+ * idle that runs of one pay, behind 256 rows already (384 from nine tiles on: 64 tokens of 28 heads over
+ * 4 behind 257 rows 14.5 us unsplit, 16.5 in three slices; append and attention, caches from HBM: 5 tokens of
+ * 28 heads over 4 of 128 behind 500 rows 10.6 us in four slices, 11.7 in two, 12.5 unsplit; 24
+ * behind 1000 rows 16.0 in eight and 16.7 in four; 73 of 14 over 2 of 64 behind 1024 12.3 and 13.3;
+ * in the mean over three shapes and prefixes to 32,768 at most 1.5 % behind the best cut, runs of two
+ * 6 % at four tiles, 3 to 6 at eight, 1 to 2 at sixteen; 256 tokens of 28 heads over 4 behind none or
+ * 256: 17.1 us unsplit, 19.6 split).
+ * `exact`: `len` is the prefix, not the capacity of a cache. */
 inline int chunk_slices(int sm_count, long long tiles, int len, bool exact) {
-  const bool ones = tiles <= 8;
-  if (tiles <= 0 || tiles * 2 > sm_count || len <= (ones ? 256 : 512)) return 1;
+  const bool ones = tiles <= (exact ? 16 : 8);
+  const int least = !ones ? 512 : tiles > 8 ? 384 : 256;
+  if (tiles <= 0 || tiles * 2 > sm_count || len <= least) return 1;
   long long s = sm_count / tiles;
   const int kv_tiles = (len + kKvTile - 1) / kKvTile;
   const int most = kv_tiles / (ones ? 1 : 2);
