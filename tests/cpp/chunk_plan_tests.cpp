@@ -58,10 +58,19 @@ static void query_tiles_are_the_kernels_own() {
   CHECK(query_tiles(3, 64) == 2, "two tokens fill one");
 }
 
+/* the capacity of a cache says little about the prefix: no runs of single tiles */
+static void a_capacity_is_cut_into_runs_of_two_tiles_at_least() {
+  for (int tiles : {1, 2, 4, 8, 16, 32, 74})
+    for (int cap : {128, 512, 513, 2048, 8192, 32768})
+      CHECK(chunk_slices(kSms, tiles, cap, false) == 1 || chunk_slices(kSms, tiles, cap, false) * 2 <= up(cap, kKvTile),
+            "%d tiles, %d rows", tiles, cap);
+}
+
 int main() {
   slices_cover_the_prefix_and_none_is_empty();
   a_prefix_that_ends_with_a_tile_is_cut_like_its_neighbours();
   query_tiles_are_the_kernels_own();
+  a_capacity_is_cut_into_runs_of_two_tiles_at_least();
   std::printf(failures ? "%d failures\n" : "chunk plan ok\n", failures);
   return failures != 0;
 }
