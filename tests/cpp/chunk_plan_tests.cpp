@@ -66,11 +66,23 @@ static void a_capacity_is_cut_into_runs_of_two_tiles_at_least() {
             "%d tiles, %d rows", tiles, cap);
 }
 
+/* few query rows: the row blocks keep what they stream faster */
+static void few_rows_go_where_they_are_faster() {
+  for (int len : {2, 128, 300, 2000, 4103, 32768}) {
+    CHECK(!chunk_in_tiles(7, 128, len) && !chunk_in_tiles(16, 128, len), "one block, len %d", len);
+    CHECK(chunk_in_tiles(35, 128, len) && chunk_in_tiles(63, 128, len), "three and four blocks, len %d", len);
+    CHECK(!chunk_in_tiles(14, 64, len) && chunk_in_tiles(28, 64, len) == (len <= 128), "64 columns, len %d", len);
+    CHECK(chunk_in_tiles(28, 128, len) == (len <= 256 || len > 2048), "two blocks, len %d", len);
+    CHECK(chunk_in_tiles(56, 64, len) == (len <= 256 || len > 2048), "four of 64 columns, len %d", len);
+  }
+}
+
 int main() {
   slices_cover_the_prefix_and_none_is_empty();
   a_prefix_that_ends_with_a_tile_is_cut_like_its_neighbours();
   query_tiles_are_the_kernels_own();
   a_capacity_is_cut_into_runs_of_two_tiles_at_least();
+  few_rows_go_where_they_are_faster();
   std::printf(failures ? "%d failures\n" : "chunk plan ok\n", failures);
   return failures != 0;
 }

@@ -543,6 +543,23 @@ def test_paged_prompts_beside_drafts(shape, lengths, counts):
         assert_close_per_head(got[cu_np[s]:cu_np[s + 1]], want, f"seq {s} ({L} + {c} rows)")
 
 
+@pytest.mark.parametrize("n_q,n_kv,hd,end,n", [(28, 4, 128, 1000, 2), (28, 4, 128, 600, 4), (32, 8, 128, 2000, 8),
+                                               (14, 2, 64, 3000, 4), (14, 2, 64, 1500, 9)])
+def test_few_rows_of_a_chunk_are_taken_by_the_row_blocks(n_q, n_kv, hd, end, n):
+    """Where they are the faster kernel: the same bits as that kernel asked for by name."""
+    rng = np.random.default_rng(end + n)
+    cache = decode.KvCache(n_kv, n_q, hd, end)
+    cache.k[:], cache.v[:] = dev(rand16(rng, (n_kv, end, hd))), dev(rand16(rng, (n_kv, end, hd)))
+    qd = dev(workloads.f16_values(rng, (n, (n_q + 2 * n_kv) * hd)))
+    outs = []
+    for choice in (0, 2):
+        check(lib.wst_b200_set_kernel_choice(choice))
+        outs.append(torch.zeros(n * n_q * hd, dtype=torch.float16, device="cuda"))
+        chunk.attn(qd, cache, outs[-1], n_q, end - n, n)
+    check(lib.wst_b200_set_kernel_choice(0))
+    assert torch.equal(outs[0], outs[1])
+
+
 def test_outputs_on_an_eight_byte_boundary():
     """Buffers that the tensor-core tiles' 16-byte stores cannot take: drafts of one sequence and
     a paged step with a prompt give what they give into aligned ones."""

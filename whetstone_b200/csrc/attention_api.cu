@@ -509,16 +509,12 @@ extern "C" wst_status_t wst_attn_chunk(const void *qkv, const void *k_cache,
   const bool tc_ok = choice != 1 && rows_kernel_supports(n_q, n_kv, head_dim, k_cache, v_cache) &&
                      aligned16(qkv);
 
-  /* 128-row tcgen05 tiles, cut along the prefix where they do not fill the GPU.  They are
-   * ahead even where most of their rows are empty: 2 tokens behind 4099 rows 10.8 us with the
-   * append against 14.3 with the mma.sync row-block kernel, 5 tokens 12.1 and 19.3 (28 heads
-   * over 4 of 128).  A single 16-row block streams better where the prefix is short (2 tokens
-   * behind 300 rows: 8.2 against 9.8) and at head_dim 64 (7.7 against 8.0); it also takes what
-   * the tiles' 16-byte stores cannot, `out` on a smaller boundary. */
+  /* 128-row tcgen05 tiles, cut along the prefix where they do not fill the GPU; of fewer rows than
+   * half a tile those that the row blocks do not stream faster.  (`out` on a smaller boundary than
+   * the tiles' 16-byte stores goes to the row blocks, which take it.) */
   const bool many = prefill_kernel_supports(n_q, n_kv, head_dim, n); /* at least 64 query rows */
-  const bool one_block = static_cast<long long>(n) * (n_q / n_kv) <= 16;
-  const bool few_in_tiles = choice == 0 && aligned16(out) &&
-                            (!one_block || (head_dim == 128 && pos0 + n > 512));
+  const bool few_in_tiles =
+      !many && choice == 0 && aligned16(out) && chunk_in_tiles(n * (n_q / n_kv), head_dim, pos0 + n);
   const bool use_prefill = tc_ok && choice != 2 && (many || few_in_tiles);
   int splits = 1;
   if (use_prefill && choice != 3 && choice != 4) {

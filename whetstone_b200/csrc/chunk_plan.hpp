@@ -50,4 +50,22 @@ inline int chunk_slices(int sm_count, long long tiles, int len, bool exact) {
   return (kv_tiles + each - 1) / each; /* no slice without a tile */
 }
 
+/* Does a chunk of fewer than 64 query rows per KV head (`rows` = tokens x heads of the group) go to
+ * the 128-row tcgen05 tiles, cut along the prefix, or to the mma.sync row-block kernel, 16 rows per
+ * block?  What a block costs goes with rows x head_dim, a tile costs the same however empty it is.
+ * Append and attention, caches from HBM, tiles against row blocks:
+ *   one block of 128 columns or two of 64: 1 token of 28 heads over 4 of 128 behind 300, 2000 and
+ *     16384 rows 8.1, 8.1 and 13.8 us against 5.9, 7.2 and 13.4; 4 of 14 over 2 of 64 behind 2000
+ *     10.1 and 8.6.  Behind a single KV tile, which needs no merge, 3 tokens of 64 columns 6.9 and 7.4;
+ *   up to twice that: 4 of 28 over 4 behind 300, 2000 and 4103 rows 10.6, 11.4 and 11.7 against
+ *     10.2, 10.8 and 12.7; behind 128 rows 8.2 and 9.4;
+ *   more (head_dim 128): 5 of 28 over 4 behind 300, 2000 and 16384 rows 10.9, 11.8 and 17.7 against
+ *     12.3, 13.0 and 27.0. */
+inline bool chunk_in_tiles(int rows, int hd, int len) {
+  const int cells = rows * hd;
+  if (cells <= 16 * 128) return rows > 16 && len <= kKvTile;
+  if (cells <= 32 * 128) return len <= 2 * kKvTile || len > 2048;
+  return true;
+}
+
 }  // namespace wst
