@@ -75,6 +75,8 @@ static void few_rows_go_where_they_are_faster() {
     CHECK(chunk_in_tiles(28, 128, len) == (len <= 256 || len > 2048), "two blocks, len %d", len);
     CHECK(chunk_in_tiles(56, 64, len) == (len <= 256 || len > 2048), "four of 64 columns, len %d", len);
   }
+  CHECK(!prompts_in_items(633, 25) && !prompts_in_items(890, 50) && prompts_in_items(891, 50), "short contexts");
+  CHECK(prompts_in_items(768, 700) && !prompts_in_items(600, 1500) && prompts_in_items(600, 1501), "long prompts");
 }
 
 int main() {

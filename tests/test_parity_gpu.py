@@ -543,6 +543,39 @@ def test_paged_prompts_beside_drafts(shape, lengths, counts):
         assert_close_per_head(got[cu_np[s]:cu_np[s + 1]], want, f"seq {s} ({L} + {c} rows)")
 
 
+# contexts of about 900 rows and more: the persistent tcgen05 kernel; all shorter: the row blocks
+@pytest.mark.parametrize("shape,lengths,counts", [
+    (workloads.QWEN25_7B, [130, 0, 1100, 61], [18, 37, 4, 19]),
+    (workloads.QWEN25_7B, [0, 1020], [129, 5]),
+    (workloads.QWEN25_05B, [300, 0, 40, 1023], [2, 130, 55, 20]),
+    (workloads.QWEN3_8B, [0, 513, 1090], [65, 5, 32]),
+])
+def test_paged_prompts_beside_drafts_and_a_longer_context(shape, lengths, counts):
+    test_paged_prompts_beside_drafts(shape, lengths, counts)
+
+
+def test_short_paged_prompts_are_taken_by_the_row_blocks():
+    """Short contexts with a prompt of two query tiles: the same bits as the
+    row-block kernel asked for by name."""
+    shape, lengths, counts = workloads.QWEN25_7B, [600, 200, 90], [3, 40, 1]
+    n_q, n_kv, hd = shape.n_q, shape.n_kv, shape.head_dim
+    rng = np.random.default_rng(11)
+    cache, _, _, _ = build_paged_case(rng, shape, lengths, max(counts))
+    total, max_len = sum(counts), max(l + c for l, c in zip(lengths, counts))
+    qd = dev(workloads.f16_values(rng, (total, shape.qkv_width)))
+    pos0, cu = dev(np.asarray(lengths, np.int32)), dev(np.concatenate([[0], np.cumsum(counts)]).astype(np.int32))
+    paged.rope_cache(qd, cache, decode.RopeTable(max_len, hd, 1e6), n_q, pos0, cu, total)
+    scratch = torch.empty(paged.verify_scratch_floats(3, max(counts), n_q, n_kv, hd, max_len),
+                          dtype=torch.float32, device="cuda")
+    outs = []
+    for choice in (0, 2):
+        check(lib.wst_b200_set_kernel_choice(choice))
+        outs.append(torch.zeros(total * n_q * hd, dtype=torch.float16, device="cuda"))
+        paged.attn_verify(qd, cache, outs[-1], scratch, n_q, pos0, cu, total, max(counts), max_len)
+    check(lib.wst_b200_set_kernel_choice(0))
+    assert torch.equal(outs[0], outs[1])
+
+
 @pytest.mark.parametrize("n_q,n_kv,hd,end,n", [(28, 4, 128, 1000, 2), (28, 4, 128, 600, 4), (32, 8, 128, 2000, 8),
                                                (14, 2, 64, 3000, 4), (14, 2, 64, 1500, 9)])
 def test_few_rows_of_a_chunk_are_taken_by_the_row_blocks(n_q, n_kv, hd, end, n):

@@ -717,13 +717,16 @@ extern "C" wst_status_t wst_attn_verify_paged(const void *qkv, const void *k_poo
    * of 128 query rows) -- its scratch layout and the merge's grid can hold: beside drafts
    * that verify, prompts of any number of rows (two of 300 rows beside six of 4 drafts
    * against 512 to 8192 rows, 28 heads over 4: 91 us per layer with the append, 255 when the
-   * row-block kernel served them). */
+   * row-block kernel served them), unless all contexts are short. */
   const int choice = g_kernel_choice.load();
   const bool one_tile = prefill_split_supports(n_q, n_kv, head_dim, max_tokens_per_seq);
   const long long verify_floats =
       wst_attn_verify_scratch_floats(n_seq, max_tokens_per_seq, n_q, n_kv, head_dim, max_len);
   /* (prompts with buffers on a smaller boundary stay with the row-block kernel, which takes them) */
-  const bool span = choice != 3 && (one_tile || (aligned16(out) && aligned16(scratch))) &&
+  const bool items = one_tile ||
+                     (prompts_in_items(max_len, static_cast<long long>(total_tokens) * (n_q / n_kv) / n_seq) &&
+                      aligned16(out) && aligned16(scratch));
+  const bool span = choice != 3 && items &&
                     verify_span_fits(n_seq, max_tokens_per_seq, n_q, n_kv, head_dim, verify_floats);
   if (choice != 2 && (one_tile || span)) {
     DeviceFacts facts;

@@ -68,4 +68,14 @@ inline bool chunk_in_tiles(int rows, int hd, int len) {
   return true;
 }
 
+/* Ragged paged batches with prompts of more than one query tile per KV head: the persistent tcgen05
+ * kernel pays three KV tiles' time for each (sequence, KV head, query tile) and a merge of partial
+ * rows, the row-block kernel reads K and V once per 64 rows.  Known here: the longest context and the
+ * mean of query rows per (sequence, KV head).  Layer with the append, 410 batches of up to 24
+ * sequences with 1 to 6 prompts of 16 to 512 rows, head_dim 64 and 128: below the line the row blocks
+ * take 0.80 of the time in the mean (0.59 to 1.16; 24 sequences of 211 to 633 rows, three prompts of
+ * 22: 24 and 31 us); above it the items take 0.77 in the mean (10 of 387 to 3096, four prompts of 483:
+ * 198 and 434 us) and 22 of 192 batches are 1.05 to 1.38 times as fast with row blocks. */
+inline bool prompts_in_items(int max_len, long long mean_rows) { return 5LL * max_len + mean_rows > 4500; }
+
 }  // namespace wst
