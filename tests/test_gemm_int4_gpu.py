@@ -169,7 +169,7 @@ def test_more_than_128_tokens_at_the_edges_of_the_tiles(in_f, out_f, n):
           3e-3 * max(1.0, (in_f / 896) ** 0.5), f"{in_f} x {out_f} x {n}")
 
 
-# K cut evenly, unevenly, with CTAs left without any (9 stages over 8), one stage; rows per CTA 64 and 128
+# K cut evenly, unevenly (nine stages over five CTAs), one stage; rows per CTA 64 and 128
 @pytest.mark.parametrize("in_f,out_f", [(3584, 2400), (1120, 330), (1056, 70), (128, 9000), (32, 17)])
 @pytest.mark.parametrize("n", [17, 33, 64, 65, 113, 128])
 def test_17_to_128_tokens_at_the_edges_of_the_tiles(in_f, out_f, n):

@@ -88,7 +88,7 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_consta
   const int rank = static_cast<int>(cluster_rank());
   const int row0 = static_cast<int>(blockIdx.x / csize) * ROWS;
   const int kb0 = rank * a.kb_cta;
-  const int nkb = max(0, min(a.kb_cta, a.k_blocks - kb0)); /* the last CTAs of a cluster may have none */
+  const int nkb = min(a.kb_cta, a.k_blocks - kb0); /* the last CTA of a cluster may have fewer */
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < nstage; ++i) {
@@ -198,20 +198,19 @@ gemm_narrow_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_consta
     const uint32_t acc = tmem + (static_cast<uint32_t>(warp * 32) << 16);
     float *part = reinterpret_cast<float *>(smem) + warp * 32 + lane;
     const bool used = warp * 32 + lane < ROWS;
-    const bool ok = nkb == 0 || mbar_wait(bar(ACC_FULL), 0, a.err_word, 0x804u);
-    const bool have = nkb > 0 && __all_sync(0xffffffffu, ok) != 0;
-    tc_fence_after_sync();
+    const bool ok = mbar_wait(bar(ACC_FULL), 0, a.err_word, 0x804u);
+    if (__all_sync(0xffffffffu, ok)) {
+      tc_fence_after_sync();
 #pragma unroll 1
-    for (int c0 = 0; c0 < a.cols; c0 += 16) {
-      uint32_t v[16];
-      if (have) {
+      for (int c0 = 0; c0 < a.cols; c0 += 16) {
+        uint32_t v[16];
         tmem_ld_32x16(acc + c0, v);
         tmem_ld_wait();
-      }
 #pragma unroll
-      for (int e = 0; e < 16; ++e)
-        if (used) part[(c0 + e) * ROWS] = have ? __uint_as_float(v[e]) : 0.f;
-      __syncwarp();
+        for (int e = 0; e < 16; ++e)
+          if (used) part[(c0 + e) * ROWS] = __uint_as_float(v[e]);
+        __syncwarp();
+      }
     }
   }
 
@@ -328,6 +327,7 @@ wst_status_t launch_cut(const PairGemm &g, int split) {
   a.cols = (g.n + 15) / 16 * 16;
   a.k_blocks = (g.in_f + C::BK - 1) / C::BK;
   a.kb_cta = (a.k_blocks + split - 1) / split;
+  split = (a.k_blocks + a.kb_cta - 1) / a.kb_cta; /* no CTA without a part of K */
   a.err_word = device_error_word();
   if (!a.err_word) return WST_ERR_CUDA;
   /* three stages if they fit beside as many slots, else two; the rest holds packed words */
