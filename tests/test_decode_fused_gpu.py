@@ -4,6 +4,9 @@ and the sharded form whose cross-GPU exchange runs inside the slice-merge kernel
 through the C ABI against the numpy oracle.  Semantics: cuda/attention.cu:57-193 of
 the engine; the knobs change summation order only."""
 
+import ctypes
+from pathlib import Path
+
 import numpy as np
 import pytest
 import torch
@@ -15,6 +18,7 @@ from whetstone_b200 import chunk, decode, workloads
 pytestmark = pytest.mark.gpu
 
 SPLITS, EARLY, STAGES = 1, 2, 4
+LATE_CURSOR = Path(__file__).resolve().parent / "cpp" / "bin" / "liblate_cursor.so"
 
 
 @pytest.fixture(autouse=True)
@@ -312,3 +316,32 @@ def test_chunk_call_without_a_workspace_runs_unsplit_and_says_so():
     want = orc.chunk_attention(q.astype(np.float64), k, v, pos0, 1.0 / np.sqrt(hd))
     assert_close_per_head(host(out).astype(np.float64).reshape(n, n_q, hd), want,
                           "chunk through the unsplit and the split launch")
+
+
+@pytest.mark.parametrize("before,after", [(5, 900), (900, 5), (0, 1023), (1023, 0)])
+@pytest.mark.parametrize("n_q,n_kv,hd", [(14, 2, 64), (28, 4, 128)])
+def test_the_append_follows_a_cursor_that_moves_late(n_q, n_kv, hd, before, after):
+    """The launch ahead lets the append start at once and moves the cursor 20 us later: whatever
+    the append read before then, the row, its rotation and the untouched rows are those of the
+    cursor as it is once that launch is complete."""
+    late = ctypes.CDLL(str(LATE_CURSOR)).late_cursor
+    late.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_void_p]
+    max_seq, theta = 1024, 1e6
+    rng = np.random.default_rng(after + hd)
+    table = decode.RopeTable(max_seq, hd, theta)
+    for _ in range(5):
+        cache = decode.KvCache(n_kv, n_q, hd, max_seq)
+        qkv = workloads.f16_values(rng, ((n_q + 2 * n_kv) * hd,))
+        qd, cursor = dev(qkv), decode.DeviceCursor(before)
+        torch.cuda.synchronize()
+        stream = torch.cuda.current_stream().cuda_stream
+        assert late(cursor.buf.data_ptr(), after, 40000, stream) == 0
+        decode.rope_cache(qd, cache, table, n_q, cursor)
+        torch.cuda.synchronize()
+        qr, kr, vv = orc.rope_append(qkv[None], np.array([after]), n_q, n_kv, hd, theta)
+        got_k, got_v = host(cache.k), host(cache.v)
+        assert np.abs(host(qd)[: n_q * hd] - qr.reshape(-1)).max() < 1e-5
+        assert np.abs(got_k[:, after].astype(np.float64) - kr[0]).max() < 4e-3     # an fp16 ulp below 8
+        assert np.array_equal(got_v[:, after], vv[0].astype(np.float16))
+        got_k[:, after], got_v[:, after] = 0, 0
+        assert not got_k.any() and not got_v.any()

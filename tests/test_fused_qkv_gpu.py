@@ -171,3 +171,49 @@ def test_fused_projection_with_int4_weights():
                                 (v_bits[s][:, pos], v.transpose(1, 0, 2), "v")):
             diff = np.abs(got.view(np.float16).astype(np.float64) - want)
             assert (diff <= 3e-3 * np.maximum(np.abs(want), 1.0)).all(), f"{what}, sequence {s}: {diff.max()}"
+
+
+# 120 tiles of 256 features for at most 74 clusters: the accumulators change hands; the last token tile is cut off
+@pytest.mark.parametrize("n_q,n_kv,hd,gains,bias", [(32, 8, 128, True, True), (80, 8, 64, False, True),
+                                                    (32, 8, 128, False, False)])
+def test_fused_projection_in_256_feature_tiles(n_q, n_kv, hd, gains, bias):
+    test_fused_projection_against_the_oracle(5, 220, 520, n_q, n_kv, hd, gains, bias)
+
+
+@pytest.mark.parametrize("n_seq,n,in_f,n_q,n_kv,hd,gains", [
+    (2, 140, 512, 4, 2, 64, True),      # narrow tiles of 64-column heads
+    (5, 220, 544, 32, 8, 128, True),    # 256 features, two tiles per cluster, K ends inside a stage
+    (5, 220, 544, 80, 8, 64, False),
+])
+def test_fused_int4_projection_with_a_bias(n_seq, n, in_f, n_q, n_kv, hd, gains):
+    from tests.test_gemm_int4_gpu import fast_packed_weights
+    theta, eps, max_seq = 1e6, 1e-6, 600
+    width = (n_q + 2 * n_kv) * hd
+    rng = np.random.default_rng(width + n)
+    qw, si, sb = fast_packed_weights(in_f, width, n)
+    x = rng.uniform(-1, 1, (n_seq * n, in_f)).astype(np.float16)
+    b = rng.standard_normal(width).astype(np.float16)
+    gq = (1 + 0.1 * rng.standard_normal(hd)).astype(np.float16) if gains else None
+    gk = (1 + 0.1 * rng.standard_normal(hd)).astype(np.float16) if gains else None
+    starts_np = rng.integers(0, max_seq - n, size=n_seq).astype(np.int32)
+    table = decode.RopeTable(max_seq, hd, theta)
+    cache = chunk.KvCacheBatch(n_seq, n_kv, hd, max_seq)
+    fill_bits(cache.k, NAN16)
+    fill_bits(cache.v, NAN16)
+    q16 = torch.zeros((n_seq * n, n_q * hd), dtype=torch.float16, device="cuda")
+    chunk.qkv_int4_rope_append_batch(dev(qw.view(np.int32)), dev(si), dev(sb.view(np.float16)), dev(x), dev(b),
+                                     q16, cache, table, n_q, dev(starts_np), n,
+                                     decode.QkNorm(dev(gq), dev(gk), eps) if gains else None)
+    torch.cuda.synchronize()
+    assert decode.device_error() == 0
+    y = orc.gemm_int4_hier(qw, si, sb, x, in_f, width, b)
+    k_bits, v_bits = bits16(cache.k), bits16(cache.v)
+    for s in range(n_seq):
+        pos = starts_np[s] + np.arange(n)
+        q_rot, k_rot, v = orc.rope_append(y[s * n:(s + 1) * n], pos, n_q, n_kv, hd, theta, gq, gk, eps)
+        for got, want, what in ((bits16(q16[s * n:(s + 1) * n]).reshape(n, n_q, hd), q_rot, "q"),
+                                (k_bits[s][:, pos], k_rot.transpose(1, 0, 2), "k"),
+                                (v_bits[s][:, pos], v.transpose(1, 0, 2), "v")):
+            diff = np.abs(got.view(np.float16).astype(np.float64) - want)
+            # as above: weights rounded to fp16 once, at about this length
+            assert (diff <= 3e-3 * np.maximum(np.abs(want), 1.0)).all(), f"{what}, sequence {s}: {diff.max()}"

@@ -142,7 +142,7 @@ def test_bad_arguments_launch_nothing():
 def test_few_tokens_at_the_edges_of_the_tiles(in_f, out_f, n):
     """The kernel for at most 32 tokens: token tiles of 8, 16 and 32 either side of their
     edges, one group of K, a slab of K that ends inside its four groups, K shorter and
-    longer than the eight warps' slabs, 16- and 32-row tiles cut off at the last row."""
+    longer than the sixteen warps' slabs, 16- and 32-row tiles cut off at the last row."""
     qw, si, sb = fast_packed_weights(in_f, out_f, in_f + out_f + n)
     rng = np.random.default_rng(n + in_f)
     x = rng.uniform(-1, 1, (n, in_f)).astype(np.float16)
@@ -151,6 +151,14 @@ def test_few_tokens_at_the_edges_of_the_tiles(in_f, out_f, n):
     got, _ = run(qw, si, sb, x, b, y0, in_f, out_f, True)
     close(got, orc.gemm_int4_hier(qw, si, sb, x, in_f, out_f, b, y0),
           3e-3 * max(1.0, (in_f / 896) ** 0.5), f"{in_f} x {out_f} x {n}")
+
+
+@pytest.mark.parametrize("in_f,out_f", [(160, 4736), (160, 4737), (2112, 6160)])
+@pytest.mark.parametrize("n", [8, 9, 16])
+def test_few_tokens_of_more_rows_than_one_wave(in_f, out_f, n):
+    """Either side of 32 rows for each of 148 SMs, where 9 to 16 tokens change from one CTA of
+    sixteen warps per SM to two of eight."""
+    test_few_tokens_at_the_edges_of_the_tiles(in_f, out_f, n)
 
 
 # scale bytes that four-byte copies cannot take (3, 5 and 9 groups a row), and those they can

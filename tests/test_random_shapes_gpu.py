@@ -117,7 +117,7 @@ def test_random_small_shapes(seed):
 @pytest.mark.parametrize("seed", [11, 12])
 def test_random_large_shapes(seed):
     """Cache lengths past 32k, chunks of several query tiles, draft counts whose
-    rows exceed one 128-row tile (the row-block kernel takes those)."""
+    rows exceed one 128-row tile (several items of the persistent kernel)."""
     rng = np.random.default_rng(seed)
     for _ in range(15):
         kind = int(rng.integers(0, 3))
