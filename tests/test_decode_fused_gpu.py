@@ -5,6 +5,7 @@ through the C ABI against the numpy oracle.  Semantics: cuda/attention.cu:57-193
 the engine; the knobs change summation order only."""
 
 import ctypes
+import subprocess
 from pathlib import Path
 
 import numpy as np
@@ -324,6 +325,9 @@ def test_the_append_follows_a_cursor_that_moves_late(n_q, n_kv, hd, before, afte
     """The launch ahead lets the append start at once and moves the cursor 20 us later: whatever
     the append read before then, the row, its rotation and the untouched rows are those of the
     cursor as it is once that launch is complete."""
+    if not LATE_CURSOR.exists():
+        subprocess.run(["make", "-C", str(LATE_CURSOR.parent.parent), "bin/liblate_cursor.so"], check=True,
+                       capture_output=True)
     late = ctypes.CDLL(str(LATE_CURSOR)).late_cursor
     late.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_void_p]
     max_seq, theta = 1024, 1e6

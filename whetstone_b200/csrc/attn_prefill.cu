@@ -1180,7 +1180,8 @@ attn_verify_span_kernel(const __grid_constant__ CUtensorMap kmap,
   constexpr int PV_DONE = P_READY + 1, Q_READY = PV_DONE + 1, EPI_DONE = Q_READY + 1;
   static_assert(EPI_DONE < C::NBAR, "barrier area");
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + C::OFF_BAR + C::NBAR * 8);
-  /* where this CTA's span starts, written by warp 0: seq, kvh, tile, span, g(lo,hi) lo hi, before */
+  /* where this CTA's span starts, written by warp 0: seq, kvh, slot in the item, span, first and last
+   * global slot, the item's first slot, query tile */
   long long *walk0 = reinterpret_cast<long long *>(smem + C::OFF_XCH + 3 * 2 * 128 * 4);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;

@@ -98,7 +98,7 @@ struct Cfg {
   /* clustered: the CTA's merged rows [ROWS][HD+4] lie behind the dump */
   static constexpr int PART_BYTES = ROWS * (HD + 4) * 4;
   static constexpr int CLUSTER_STAGES = (DUMP_BYTES + PART_BYTES + STAGE_BYTES - 1) / STAGE_BYTES;
-  static_assert(MIN_STAGES <= NSTAGE, "combine buffer must fit the ring");
+  static_assert(MIN_STAGES <= NSTAGE && CLUSTER_STAGES <= NSTAGE, "combine buffer must fit the ring");
   static_assert(smem_bytes(NSTAGE) <= 232448, "shared memory of one CTA");
 };
 

@@ -5,18 +5,18 @@
  * x [n][in_f] and w [out_f][in_f] fp16, y [n][out_f] fp32 -- wst_gemm_fp16 of the
  * engine (cuda/chunk_gemm.cu:178-258, dispatch :340-365).  The engine's kernel keeps
  * the weights outermost and covers at most 16 tokens per pass; every weight row is a
- * warp's dot product in half2.  Here any number of tokens is one launch:
+ * warp's dot product in half2.  Here any number of tokens is one launch; this file's kernel
+ * takes up to 128, more go to gemm_pair.cu:
  *
  *   both operands are K-major, so a 128-token x BN-feature tile is
  *   tcgen05.mma.kind::f16 M128 x N(BN) x K16 straight from the TMA-filled,
  *   128-byte-swizzled stages (x tile 16 KB + w tile BN*128 B per 64 columns of K);
  *   fp32 accumulators in tensor memory, TWO of them, so the epilogue of one tile
  *   (tensor memory -> registers -> + bias (+ y) -> global) runs under the main loop
- *   of the next; persistent CTAs, one per SM, walk the tiles token-tile fastest so
- *   that the CTAs running at the same time share a weight tile in L2.
+ *   of the next; persistent CTAs, one per SM, walk the feature tiles.
  *
- *   BN = 32, 48 or 64: up to 128 tokens the launch is a stream of the weights, and as
- *   many CTAs as there are SMs pull on HBM.  More tokens go to gemm_pair.cu.
+ *   BN = 32, 48 or 64: the launch is a stream of the weights, and as many CTAs as there
+ *   are SMs pull on HBM.
  *
  * Products are exact in fp32 and accumulated in fp32 (the engine's kernel rounds
  * every group of four products to fp16 first): results differ from the engine's by
@@ -46,7 +46,7 @@ using namespace ptx;
  * come of it belong to tokens that do not exist and are never stored). */
 template <int BN, int KS, int RB>
 struct GCfg {
-  static constexpr int BM = 128, BK = 64 * KS;
+  static constexpr int BK = 64 * KS;
   static constexpr int A_SLAB = RB * 128, B_SLAB = BN * 128;
   static constexpr int A_BYTES = KS * A_SLAB;
   static constexpr int B_BYTES = KS * B_SLAB;
@@ -66,7 +66,7 @@ struct GemmArgs {
   const __half *bias;
   float *y;
   int in_f, out_f, n, accum;
-  int m_tiles, n_tiles;
+  int n_tiles;
   unsigned int *err_word;
 };
 
@@ -112,17 +112,16 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant_
 
   grid_dependency_wait();
 
-  const int n_tiles_total = a.m_tiles * a.n_tiles;
   const int k_blocks = (a.in_f + C::BK - 1) / C::BK;
-  /* tile i of this CTA is global tile blockIdx.x + i * gridDim.x: token tile fastest */
+  /* tile i of this CTA is feature tile blockIdx.x + i * gridDim.x */
 
   if (warp == 5) {
     /* ------------------------------------------------------ TMA producer */
     if (lane == 0) {
       int it = 0; /* stage uses so far */
       bool ok = true;
-      for (int tile = blockIdx.x; ok && tile < n_tiles_total; tile += gridDim.x) {
-        const int m0 = (tile % a.m_tiles) * C::BM, n0 = (tile / a.m_tiles) * BN;
+      for (int tile = blockIdx.x; ok && tile < a.n_tiles; tile += gridDim.x) {
+        const int n0 = tile * BN;
         for (int kb = 0; kb < k_blocks; ++kb, ++it) {
           const int st = it % NSTAGE;
           if (it >= NSTAGE &&
@@ -132,11 +131,11 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant_
           }
           mbar_arrive_expect_tx(bar(FULL + st), C::STAGE_BYTES);
           if constexpr (KS == 1) { /* maps over [rows][in_f]: columns past in_f read as zero */
-            tma_load_3d(sbase + st * C::STAGE_BYTES, &xmap, bar(FULL + st), kb * C::BK, m0, 0);
+            tma_load_3d(sbase + st * C::STAGE_BYTES, &xmap, bar(FULL + st), kb * C::BK, 0, 0);
             tma_load_3d(sbase + st * C::STAGE_BYTES + C::A_BYTES, &wmap, bar(FULL + st), kb * C::BK,
                         n0, 0);
           } else { /* maps over [in_f / 64][rows][64]: KS slabs per request */
-            tma_load_3d(sbase + st * C::STAGE_BYTES, &xmap, bar(FULL + st), 0, m0, kb * KS);
+            tma_load_3d(sbase + st * C::STAGE_BYTES, &xmap, bar(FULL + st), 0, 0, kb * KS);
             tma_load_3d(sbase + st * C::STAGE_BYTES + C::A_BYTES, &wmap, bar(FULL + st), 0, n0,
                         kb * KS);
           }
@@ -148,7 +147,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant_
     constexpr uint32_t idesc = umma_idesc(128, BN, 0);
     int it = 0, local = 0;
     bool ok = true;
-    for (int tile = blockIdx.x; ok && tile < n_tiles_total; tile += gridDim.x, ++local) {
+    for (int tile = blockIdx.x; ok && tile < a.n_tiles; tile += gridDim.x, ++local) {
       const int buf = local & 1;
       /* the epilogue of the tile two back has emptied this accumulator */
       if (local >= 2 &&
@@ -180,20 +179,19 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant_
     const uint32_t lane_base = static_cast<uint32_t>(warp * 32) << 16;
     const bool vec = (a.out_f & 3) == 0;
     int local = 0;
-    for (int tile = blockIdx.x; tile < n_tiles_total; tile += gridDim.x, ++local) {
+    for (int tile = blockIdx.x; tile < a.n_tiles; tile += gridDim.x, ++local) {
       const int buf = local & 1;
-      const int m0 = (tile % a.m_tiles) * C::BM, n0 = (tile / a.m_tiles) * BN;
+      const int n0 = tile * BN;
       if (!mbar_wait_idle(bar(ACC_FULL + buf), (local >> 1) & 1, a.err_word, 0x604u)) break;
       tc_fence_after_sync();
-      const int row = m0 + r;
-      float *yrow = a.y + static_cast<long long>(row) * a.out_f;
+      float *yrow = a.y + static_cast<long long>(r) * a.out_f;
 #pragma unroll 1
       for (int c0 = 0; c0 < BN; c0 += 32) {
         uint32_t v[32];
         tmem_ld_32x32(tmem + lane_base + buf * C::ACC_STRIDE + c0, v);
         tmem_ld_wait();
         const int col0 = n0 + c0;
-        if (row < a.n && col0 < a.out_f) {
+        if (r < a.n && col0 < a.out_f) {
           if (vec && c0 + 32 <= BN && col0 + 32 <= a.out_f) {
 #pragma unroll
             for (int e = 0; e < 32; e += 4) {
@@ -265,17 +263,7 @@ gemm_f16_plain_kernel(const __half *w, const __half *x, const __half *bias, floa
  * row, column -- so that one request brings KS slabs. */
 wst_status_t operand_map(CUtensorMap *out, const void *base, int in_f, int rows, int box_rows,
                          int ks) {
-  if (ks == 1) {
-    KvMapKey key{};
-    key.rank = 3;
-    key.base = base;
-    key.d0 = static_cast<uint64_t>(in_f);
-    key.d1 = static_cast<uint64_t>(rows);
-    key.d2 = 1;
-    key.d3 = 1;
-    key.b1 = static_cast<uint32_t>(box_rows);
-    return cached_kv_tensor_map(out, key);
-  }
+  if (ks == 1) return rows_map(out, base, in_f, rows, box_rows);
   struct Slot {
     const void *base;
     int in_f, rows, box_rows, ks;
@@ -315,11 +303,9 @@ wst_status_t launch_gemm(const void *w, const void *x, GemmArgs a, int sm_count)
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
     configured_dev = dev;
   }
-  a.m_tiles = (a.n + C::BM - 1) / C::BM;
   a.n_tiles = (a.out_f + BN - 1) / BN;
-  const long long tiles = static_cast<long long>(a.m_tiles) * a.n_tiles;
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(static_cast<unsigned>(tiles < sm_count ? tiles : sm_count));
+  cfg.gridDim = dim3(static_cast<unsigned>(a.n_tiles < sm_count ? a.n_tiles : sm_count));
   cfg.blockDim = dim3(kGemmThreads);
   cfg.dynamicSmemBytes = C::SMEM_BYTES;
   cfg.stream = current_stream();

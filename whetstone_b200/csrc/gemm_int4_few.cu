@@ -25,6 +25,7 @@
  * rounded to fp16 once; products and sums fp32. */
 
 #include "gemm_int4_few.cuh"
+#include "int4_tile.cuh"
 #include "wst_ptx.cuh"
 
 namespace wst {
@@ -112,19 +113,12 @@ __global__ void __launch_bounds__(32 * WARPS, 16 / WARPS) gemm_int4_few_kernel(c
                            : make_uint4(0u, 0u, 0u, 0u);
   };
   /* word `wi` of the rows' groups: unpacked, multiplied */
-  auto multiply = [&](const Slab<MT> &d, const float (&sc)[RI], const float (&mn)[RI], int wi,
-                      const uint4 (&x)[NT]) {
+  auto multiply = [&](const Slab<MT> &d, const GroupScale (&sc)[RI], int wi, const uint4 (&x)[NT]) {
     uint32_t o[RI][4]; /* the word's weights 2i, 2i + 1 as fp16 */
 #pragma unroll
     for (int i = 0; i < RI; ++i) {
       const uint32_t word = wi == 0 ? d.w[i].x : wi == 1 ? d.w[i].y : wi == 2 ? d.w[i].z : d.w[i].w;
-      const uint32_t even = word & 0x0F0F0F0Fu, odd = (word >> 4) & 0x0F0F0F0Fu;
-#pragma unroll
-      for (int b = 0; b < 4; ++b) { /* nibble into byte 2 of 0.5f: 0.5 + q / 256 */
-        const float f0 = __uint_as_float(__byte_perm(even, 0x3F000000u, 0x7044u | (b << 8)));
-        const float f1 = __uint_as_float(__byte_perm(odd, 0x3F000000u, 0x7044u | (b << 8)));
-        o[i][b] = pack_half2(fmaf(f0, sc[i], mn[i]), fmaf(f1, sc[i], mn[i]));
-      }
+      unpack_word(word, sc[i], o[i]);
     }
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt) {
@@ -152,17 +146,13 @@ __global__ void __launch_bounds__(32 * WARPS, 16 / WARPS) gemm_int4_few_kernel(c
       if (s + h * WARPS >= slabs) break;
       fetch(s + (h + 1) * WARPS, buf[h ^ 1]);
       const Slab<MT> &d = buf[h];
-      float sc[RI], mn[RI];
+      GroupScale sc[RI];
 #pragma unroll
-      for (int i = 0; i < RI; ++i) {
-        const float s1 = dd[i].x * static_cast<float>(d.idx[i] & 0xF); /* d * ls */
-        sc[i] = 256.0f * s1;
-        mn[i] = fmaf(-128.0f, s1, -dd[i].y * static_cast<float>(d.idx[i] >> 4));
-      }
+      for (int i = 0; i < RI; ++i) sc[i] = group_scale(dd[i], d.idx[i]);
 #pragma unroll
       for (int wi = 0; wi < 4; ++wi) {
         const int p = 4 * h + wi, next = p + RING;
-        multiply(d, sc, mn, wi, xb[p % RING]);
+        multiply(d, sc, wi, xb[p % RING]);
         fetch_x(s + (next >> 2) * WARPS, next & 3, xb[p % RING]);
       }
     }

@@ -74,12 +74,6 @@ struct PairArgs {
 
 /* ---- two-CTA forms of the tcgen05 and mbarrier instructions */
 
-/* the same shared-memory offset in the pair's first CTA */
-__device__ __forceinline__ uint32_t in_leader(uint32_t addr) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(addr));
-  return r;
-}
 /* Tells the pair's first CTA, by 16 bytes that its barrier counts, that what this thread has seen
  * happen in its own CTA has happened: the copy is issued behind that, and its completion is a
  * release at cluster scope.  (An arrival with such a release is as sound but makes the arriving
@@ -89,7 +83,7 @@ constexpr int kMessage = 16;
 __device__ __forceinline__ void tell_leader(uint32_t mailbox, uint32_t src, uint32_t bar) {
   asm volatile(
       "cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-      ::"r"(in_leader(mailbox)), "r"(src), "n"(kMessage), "r"(in_leader(bar))
+      ::"r"(in_cta(mailbox, 0)), "r"(src), "n"(kMessage), "r"(in_cta(bar, 0))
       : "memory");
 }
 __device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity) {
@@ -177,7 +171,7 @@ __device__ __forceinline__ void add_v4(float *y, float4 v) {
  * row; v heads are narrowed and stored as they are.  The arithmetic is that of
  * rope_append_kernel (norm before rotation, x * inv * gain, cuda/decode.cu:112-178 and
  * cuda/chunk_ops.cu:101-150 of the engine).  The head is read twice, once for the norm and
- * then sixteen column pairs at a time: 704 threads leave 88 registers. */
+ * then sixteen column pairs at a time: 736 threads leave 80 registers. */
 template <int HD>
 __device__ __forceinline__ void rope_head_epilogue(const PairGemm &g, uint32_t tmem_head, int head,
                                                    int tpos, long long kv_row, int tok, bool valid) {
@@ -351,7 +345,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant
            * CTA's weights are unpacked */
           if (rank == 0)
             mbar_arrive_expect_tx(bar(FULL + st), INT4 ? 2 * C::A_BYTES + kMessage : 2 * C::STAGE_BYTES);
-          const uint32_t full = in_leader(bar(FULL + st));
+          const uint32_t full = in_cta(bar(FULL + st), 0);
           const uint32_t dst = sbase + st * C::STAGE_BYTES;
 #pragma unroll
           for (int s = 0; s < C::KS; ++s) {

@@ -69,37 +69,48 @@ struct PackedRows {
 /* before the fetching warp leaves: its own copies have landed */
 __device__ __forceinline__ void fetch_packed_drain() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-/* Group j (32 columns) of `row` of a ROWS-row slot -> fp16 weights in the operand tile of two
- * 64-column slabs at `tile`.  Eight rows x four groups per warp: lane = 4 (row % 8) + j.
- * A nibble q dropped into byte 2 of 0x3F000000 is the float 0.5 + q / 256, one byte permute
+/* A nibble q dropped into byte 2 of 0x3F000000 is the float 0.5 + q / 256, one byte permute
  * per weight; then w = q s - dmin lm = (256 s) f - (128 s + dmin lm) with s = d * ls is ONE fp32
  * fma per weight, and the result is rounded to fp16 once -- the only difference from the exact
  * weight, random in sign.  (In half2 arithmetic the rounded offset is common to the 32 weights
  * of a group and adds up along it: 9.7e-3 from the exact product on the engine's test case
- * where this form has 1.3e-3.)  Columns past in_f came as zeros and meet zeros of x. */
+ * where this form has 1.3e-3.) */
+struct GroupScale {
+  float mul, add; /* 256 s, -(128 s + dmin lm) */
+};
+__device__ __forceinline__ GroupScale group_scale(float2 dd, unsigned idx) {
+  const float s1 = dd.x * static_cast<float>(idx & 0xFu); /* d * ls */
+  return {256.0f * s1, fmaf(-128.0f, s1, -dd.y * static_cast<float>(idx >> 4))};
+}
+/* the eight weights of a word, 2i (low nibble of byte i) and 2i + 1 as one half2 */
+__device__ __forceinline__ void unpack_word(uint32_t word, GroupScale g, uint32_t (&o)[4]) {
+  const uint32_t even = word & 0x0F0F0F0Fu, odd = (word >> 4) & 0x0F0F0F0Fu;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float f0 = __uint_as_float(__byte_perm(even, 0x3F000000u, 0x7044u | (i << 8)));
+    const float f1 = __uint_as_float(__byte_perm(odd, 0x3F000000u, 0x7044u | (i << 8)));
+    o[i] = ptx::pack_half2(fmaf(f0, g.mul, g.add), fmaf(f1, g.mul, g.add));
+  }
+}
+
+/* Group j (32 columns) of `row` of a ROWS-row slot -> fp16 weights in the operand tile of two
+ * 64-column slabs at `tile`.  Eight rows x four groups per warp: lane = 4 (row % 8) + j.
+ * Columns past in_f came as zeros and meet zeros of x. */
 template <int ROWS>
 __device__ __forceinline__ void unpack_group(const uint8_t *slot, uint8_t *tile, int row, int j, float2 dd) {
   using namespace ptx;
   const uint4 w = *reinterpret_cast<const uint4 *>(slot + row * 64 + j * 16);
   const unsigned idx = slot[ROWS * 64 + row * 4 + j];
   uint8_t *slab = tile + (j >> 1) * ROWS * 128;
-  const float s1 = dd.x * static_cast<float>(idx & 0xFu); /* d * ls */
-  const float sc = 256.0f * s1;
-  const float mt = fmaf(-128.0f, s1, -dd.y * static_cast<float>(idx >> 4));
+  const GroupScale scale = group_scale(dd, idx);
   /* the two slabs' lanes take their words in different order: the eight 16-byte stores of a
    * phase, two rows x four groups, then fall on eight different bank groups */
   const bool swap = j >= 2;
   const uint32_t words[4] = {swap ? w.z : w.x, swap ? w.w : w.y, swap ? w.x : w.z, swap ? w.y : w.w};
 #pragma unroll
   for (int wi = 0; wi < 4; ++wi) { /* 8 weights = one 16-byte chunk per word */
-    const uint32_t even = words[wi] & 0x0F0F0F0Fu, odd = (words[wi] >> 4) & 0x0F0F0F0Fu;
     uint32_t o[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) { /* weights 2i (low nibble of byte i) and 2i + 1 */
-      const float f0 = __uint_as_float(__byte_perm(even, 0x3F000000u, 0x7044u | (i << 8)));
-      const float f1 = __uint_as_float(__byte_perm(odd, 0x3F000000u, 0x7044u | (i << 8)));
-      o[i] = pack_half2(fmaf(f0, sc, mt), fmaf(f1, sc, mt));
-    }
+    unpack_word(words[wi], scale, o);
     const int chunk = (j & 1) * 4 + (swap ? wi ^ 2 : wi);
     *reinterpret_cast<uint4 *>(slab + swz128(row, chunk)) = make_uint4(o[0], o[1], o[2], o[3]);
   }

@@ -241,22 +241,6 @@ __device__ __forceinline__ float ex2(float x) {
   return y;
 }
 
-/* 2^x on the FMA and integer pipes instead of the special-function unit (which
- * delivers 16 results per clock and SM and is what bounds a softmax over
- * 128-wide tiles).  round-to-nearest split x = n + f, f in [-0.5, 0.5]; a cubic
- * for 2^f (minimax in relative error, 7.5e-5 -- below half an fp16 ulp of the
- * probability it becomes); n is added into the exponent field.  x is clamped at
- * -125, so -inf (a masked score) gives 2^-125, which rounds to 0 in fp16. */
-__device__ __forceinline__ float ex2_fma(float x) {
-  x = fmaxf(x, -125.f);
-  const float t = x + 12582912.f; /* 1.5 * 2^23: round(x) lands in the low mantissa bits */
-  const float f = x - (t - 12582912.f);
-  float p = fmaf(0.0551716685f, f, 0.2426111251f);
-  p = fmaf(p, f, 0.6932609677f);
-  p = fmaf(p, f, 0.9999280572f);
-  return __int_as_float(__float_as_int(p) + (__float_as_int(t) << 23));
-}
-
 /* --------------------------------------------------------------- tcgen05 */
 
 /* Allocates `cols` (power of two, 32..512) tensor-memory columns; one full warp
