@@ -28,8 +28,9 @@ static void slices_cover_the_prefix_and_none_is_empty() {
     for (int n_kv : {1, 2, 4, 8, 32})
       for (int n : {1, 2, 5, 9, 18, 19, 64, 73, 128, 256, 512})
         for (int len = n; len <= 40000; len = len < 1100 ? len + 1 : len + 61) {
+          const int hd = len % 2 ? 64 : 128;
           const long long tiles = query_tiles(n, gqa) * n_kv;
-          const int s = chunk_slices(kSms, tiles, len, true);
+          const int s = chunk_slices(kSms, tiles, hd, len, true);
           if (s == 1) continue;
           const int kv = up(len, kKvTile), each = slice_tiles(len, s);
           CHECK(s <= kMaxChunkSlices && s * tiles <= kSms, "%d slices of %lld tiles", s, tiles);
@@ -41,12 +42,13 @@ static void slices_cover_the_prefix_and_none_is_empty() {
 static void a_prefix_that_ends_with_a_tile_is_cut_like_its_neighbours() {
   for (int tiles : {1, 2, 4, 8})
     for (int len = 512; len <= 4096; len += 128) {
-      const int s = chunk_slices(kSms, tiles, len, true);
-      CHECK(s == chunk_slices(kSms, tiles, len - 1, true), "len %d", len);
+      const int hd = len % 256 ? 128 : 64;
+      const int s = chunk_slices(kSms, tiles, hd, len, true);
+      CHECK(s == chunk_slices(kSms, tiles, hd, len - 1, true), "len %d", len);
       CHECK(slice_tiles(len, s) == slice_tiles(len - 1, s), "len %d", len);
     }
   /* 28 heads over 4, 5 tokens, 4096 positions: 32 KV tiles in 32 slices */
-  const int s = chunk_slices(kSms, query_tiles(5, 7) * 4, 4096, true);
+  const int s = chunk_slices(kSms, query_tiles(5, 7) * 4, 128, 4096, true);
   CHECK(s == 32 && slice_tiles(4096, s) == 1, "%d slices of %d", s, slice_tiles(4096, s));
 }
 
@@ -62,7 +64,7 @@ static void query_tiles_are_the_kernels_own() {
 static void a_capacity_is_cut_into_runs_of_two_tiles_at_least() {
   for (int tiles : {1, 2, 4, 8, 16, 32, 74})
     for (int cap : {128, 512, 513, 2048, 8192, 32768})
-      CHECK(chunk_slices(kSms, tiles, cap, false) == 1 || chunk_slices(kSms, tiles, cap, false) * 2 <= up(cap, kKvTile),
+      CHECK(chunk_slices(kSms, tiles, 128, cap, false) == 1 || chunk_slices(kSms, tiles, 128, cap, false) * 2 <= up(cap, kKvTile),
             "%d tiles, %d rows", tiles, cap);
 }
 

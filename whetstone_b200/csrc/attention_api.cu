@@ -520,7 +520,7 @@ extern "C" wst_status_t wst_attn_chunk(const void *qkv, const void *k_cache,
   if (use_prefill && choice != 3 && choice != 4) {
     DeviceFacts facts;
     if (!device_facts(&facts)) return WST_ERR_CUDA;
-    splits = chunk_slices(facts.sm_count, query_tiles(n, n_q / n_kv) * n_kv, pos0 + n, true);
+    splits = chunk_slices(facts.sm_count, query_tiles(n, n_q / n_kv) * n_kv, head_dim, pos0 + n, true);
   }
   if (use_prefill) {
     PrefillLaunch P;
@@ -616,7 +616,7 @@ static wst_status_t chunk_batch_common(const void *qkv, bool q16, const void *k_
       DeviceFacts facts;
       if (!device_facts(&facts)) return WST_ERR_CUDA;
       const int splits =
-          chunk_slices(facts.sm_count, query_tiles(n, n_q / n_kv) * n_kv * n_seq, max_seq, false);
+          chunk_slices(facts.sm_count, query_tiles(n, n_q / n_kv) * n_kv * n_seq, head_dim, max_seq, false);
       if (splits > 1) {
         const char *why = "";
         P.scratch = chunk_workspace(&why);

@@ -1458,10 +1458,10 @@ wst_status_t launch_split_merge(const SplitMerge &S) {
   if (!m.err_word) return WST_ERR_CUDA;
   cudaError_t e;
   /* few slices, many rows (ragged verify, a sliced chunk): a warp per row, eight slices at once.
-   * Nine to sixteen take it two rounds, which only many units pay for: append, attention and merge
-   * of a chunk of up to eight units 0.98, 0.97 and 0.96 of the time with a block per row at 10, 12
-   * and 16 slices, 1.01 at 2 to 8; of nine to sixteen units 1.04 and 1.03 at 10 and 12. */
-  const int warp_slices = S.n_units > 8 ? 16 : 8;
+   * Nine to sixteen take it two rounds, which only many rows pay for: append, attention and merge of
+   * a chunk with a block per row take 0.96 of the time with a warp per row at 10 to 16 slices of up to
+   * 600 rows in all (1.00 at 2 to 8), 1.03 at 10 and 12 of up to 1100, 1.05 and 1.03 of more. */
+  const int warp_slices = static_cast<long long>(S.n_units) * S.rows_cap > 600 ? 16 : 8;
   if ((S.slice_counts || (S.n_splits <= warp_slices && S.rows_cap >= 16)) && !S.partial_out && S.world <= 1) {
     const dim3 rgrid(static_cast<unsigned>((S.rows_cap + 7) / 8), static_cast<unsigned>(S.n_units));
     e = S.hd == 128 ? launch_pdl(attn_merge_rows_kernel<128>, rgrid, dim3(256), 0, 1, m)

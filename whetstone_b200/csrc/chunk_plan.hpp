@@ -32,7 +32,7 @@ inline int slice_tiles(int len, int slices) {
  * `exact`: every query tile sees about `len`.  Where it is only the capacity of the caches a short
  * prefix pays for every slice that finds nothing: 16 tokens behind 200 rows in a cache of 2048 take
  * 11.3 us in sixteen slices and 10.5 in eight, and behind 1000 rows the two are level. */
-inline int chunk_slices(int sm_count, long long tiles, int len, bool exact) {
+inline int chunk_slices(int sm_count, long long tiles, int hd, int len, bool exact) {
   const bool ones = exact && tiles <= 16;
   const int least = !ones ? 512 : tiles > 8 ? 384 : 256;
   if (tiles <= 0 || tiles * 2 > sm_count || len <= least) return 1;
@@ -45,8 +45,9 @@ inline int chunk_slices(int sm_count, long long tiles, int len, bool exact) {
   if (!exact) return static_cast<int>(s); /* the kernel cuts each prefix as it finds it */
   int each = slice_tiles(len, static_cast<int>(s));
   /* where runs of one would take nearly every SM the merge and the next launch find none free: 5
-   * tokens of 28 heads over 4 behind 4103 rows 13.7 us in 33 slices, 12.1 in 17 */
-  if (each == 1 && kv_tiles * tiles * 8 > sm_count * 7LL) each = 2;
+   * tokens of 28 heads over 4 of 128 behind 4103 rows 13.7 us in 33 slices, 12.1 in 17.  (Tiles of 64
+   * columns take half as long: 24 of 14 over 2 of 64 11.2 and 11.9.) */
+  if (hd == 128 && each == 1 && kv_tiles * tiles * 8 > sm_count * 7LL) each = 2;
   return (kv_tiles + each - 1) / each; /* no slice without a tile */
 }
 
