@@ -1460,8 +1460,10 @@ wst_status_t launch_split_merge(const SplitMerge &S) {
   /* few slices, many rows (ragged verify, a sliced chunk): a warp per row, eight slices at once.
    * Nine to sixteen take it two rounds, which only many rows pay for: append, attention and merge of
    * a chunk with a block per row take 0.96 of the time with a warp per row at 10 to 16 slices of up to
-   * 600 rows in all (1.00 at 2 to 8), 1.03 at 10 and 12 of up to 1100, 1.05 and 1.03 of more. */
-  const int warp_slices = static_cast<long long>(S.n_units) * S.rows_cap > 600 ? 16 : 8;
+   * 600 rows in all (1.00 at 2 to 8), at 600 to 1100 rows 1.02 at 10 and 12 slices and 1.00 (0.93 to
+   * 1.04) at 16, with more rows 1.05 and 1.03 at 10 and 12. */
+  const long long rows = static_cast<long long>(S.n_units) * S.rows_cap;
+  const int warp_slices = rows > 1100 ? 16 : rows > 600 ? 12 : 8;
   if ((S.slice_counts || (S.n_splits <= warp_slices && S.rows_cap >= 16)) && !S.partial_out && S.world <= 1) {
     const dim3 rgrid(static_cast<unsigned>((S.rows_cap + 7) / 8), static_cast<unsigned>(S.n_units));
     e = S.hd == 128 ? launch_pdl(attn_merge_rows_kernel<128>, rgrid, dim3(256), 0, 1, m)
