@@ -265,6 +265,8 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
           if (8 * kb + (lane >> 2) >= live) w[n][0] = w[n][1] = w[n][2] = w[n][3] = 0u;
         }
         if (use > 0 && !mbar_wait(bar(C_EMPTY + cs), (use - 1) & 1, a.err_word, 0x703u)) break;
+        /* the last slot held the query rows on their way into tensor memory */
+        if (j == C::NV - 1 && !mbar_wait(bar(Q_READY), 0, a.err_word, 0x705u)) break;
 #pragma unroll
         for (int n = 0; n < 8; ++n) {
           const int kb = 4 * cw + (n >> 1);
@@ -376,20 +378,42 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_con
     const uint32_t lane_base = static_cast<uint32_t>(w * 32) << 16;
     const bool valid = lane < a.gqa;
 
-    /* q row `lane` of the group, replicated in every quadrant: fp16 * scale, two per column */
+    /* q row `lane` of the group, replicated in every quadrant: fp16 * scale, two per column.  Read
+     * whole rows at a time, a quarter of them per warp, and turned in the last V slot, which nobody
+     * writes before Q_READY: with every lane walking a row of its own in all four warps the loads
+     * were 0.45 us of each launch slower than through the read-only path, which is not for data
+     * that the launch ahead writes. */
     {
-      const float *src = a.q + static_cast<long long>(kvh * a.gqa + (valid ? lane : 0)) * HD;
+      constexpr int QROW = 2 * HD + 16; /* bytes: eight lanes' 16-byte reads on different banks */
+      const uint32_t qbuf = sbase + C::OFF_CONV + (C::NCV - 1) * C::SLOT;
+      float4 f[4];
 #pragma unroll
-      for (int c0 = 0; c0 < HD / 2; c0 += 32) {
-        uint32_t qp[32];
+      for (int k = 0; k < 4; ++k)
+        if (w + 4 * k < a.gqa)
+          f[k] = *reinterpret_cast<const float4 *>(
+              a.q + static_cast<long long>(kvh * a.gqa + w + 4 * k) * HD + 4 * lane);
 #pragma unroll
-        for (int e = 0; e < 32; e += 2) {
-          const float4 f = *reinterpret_cast<const float4 *>(src + 2 * (c0 + e));
-          qp[e] = valid ? pack_half2(f.x * a.qscale, f.y * a.qscale) : 0u;
-          qp[e + 1] = valid ? pack_half2(f.z * a.qscale, f.w * a.qscale) : 0u;
-        }
-        tmem_st_32x32(tmem + lane_base + C::COL_Q + c0, qp);
+      for (int k = 0; k < 4; ++k)
+        if (w + 4 * k < a.gqa)
+          asm volatile("st.shared.v2.b32 [%0], {%1,%2};" ::"r"(qbuf + (w + 4 * k) * QROW + 8 * lane),
+                       "r"(pack_half2(f[k].x * a.qscale, f[k].y * a.qscale)),
+                       "r"(pack_half2(f[k].z * a.qscale, f[k].w * a.qscale))
+                       : "memory");
+      asm volatile("bar.sync 1, 128;" ::: "memory");
+      uint32_t qp[HD / 2];
+#pragma unroll
+      for (int e = 0; e < HD / 2; e += 4) {
+        qp[e] = qp[e + 1] = qp[e + 2] = qp[e + 3] = 0u;
+        if (valid)
+          asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];"
+                       : "=r"(qp[e]), "=r"(qp[e + 1]), "=r"(qp[e + 2]), "=r"(qp[e + 3])
+                       : "r"(qbuf + lane * QROW + 4 * e)
+                       : "memory");
       }
+      __syncwarp();
+#pragma unroll
+      for (int c0 = 0; c0 < HD / 2; c0 += 32)
+        tmem_st_32x32(tmem + lane_base + C::COL_Q + c0, *reinterpret_cast<uint32_t(*)[32]>(&qp[c0]));
       /* this quadrant's rows of P: zero outside the stream's own keys, for good */
       uint32_t z[32];
 #pragma unroll
